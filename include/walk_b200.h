@@ -64,6 +64,9 @@ extern "C" {
 #define WALK_B200_CSR_WANT_TRIFILTER 0x8u /* walk_b200_graph_create only, with _SYMMETRIC and _WANT_EDGESET: also build the
                                              triangle filter (walk_b200_trifilter_build; tuning trifilter_max_row) */
 
+#define WALK_B200_CSR_STEPS 0x10u /* `revpos` holds the graph's step array instead (walk_b200_steps_build), `reserved` its
+                                     field widths */
+
 typedef struct walk_b200_csr {
   const int64_t* rowptr;   /* device, [num_nodes + 1] */
   const int64_t* col;      /* device, [num_edges]; node2vec needs each row sorted ascending */
@@ -109,7 +112,8 @@ const char* walk_b200_last_error(void);
 /* Number of kernels this library has launched in this process (all threads). */
 uint64_t walk_b200_launch_count(void);
 /* Name of the kernel the calling thread launched last through this library ("" before the first launch),
- * e.g. "node2vec_pool_kernel": lets a host check which variant a call selected. */
+ * e.g. "node2vec_pool_kernel": lets a host check which variant a call selected. A node2vec batch small enough for the
+ * team kernel reports the kernel that a larger batch of the same call would run. */
 const char* walk_b200_last_kernel(void);
 
 /*

@@ -14,12 +14,12 @@ PKG = Path(__file__).resolve().parent
 CSRC = PKG / "csrc"
 LIB = PKG / "libwalk_b200.so"
 SOURCES = [CSRC / "walk_b200.cu", CSRC / "csr_build.cu", CSRC / "host_widen.cpp"]
-HEADERS = [CSRC / "walk_kernels.cuh", CSRC / "philox.cuh", CSRC / "host_widen.h", CSRC / "n2v_pool.cuh", CSRC / "n2v_pool_tri.cuh", CSRC / "host_common.h", PKG.parent / "include" / "walk_b200.h"]
+HEADERS = [CSRC / "walk_kernels.cuh", CSRC / "philox.cuh", CSRC / "host_widen.h", CSRC / "n2v_pool.cuh", CSRC / "n2v_pool_tri.cuh", CSRC / "n2v_team.cuh", CSRC / "host_common.h", PKG.parent / "include" / "walk_b200.h"]
 
 NVCC_FLAGS = [
     "-gencode", "arch=compute_100a,code=sm_100a",
     "-lineinfo", "-O3", "-std=c++17",
-    "-Xcompiler", "-fPIC,-pthread", "-shared",
+    "-Xcompiler", "-fPIC,-pthread", "-shared", "--threads", "0",
     "--fmad=false",  # the uniform walk's float32 product must not be contracted
 ]
 

@@ -1,0 +1,213 @@
+// node2vec walk, team form: T lanes of a warp walk one walk together.
+//
+// A rejection step is a chain of tries, each a draw, a candidate gather and perhaps a membership test, and the
+// per-lane and pooled kernels run the tries of a step one after another. That is the right thing when millions of
+// walks keep the memory system busy. A batch of a few thousand walks leaves it idle and pays every latency in turn:
+// 2,708 walks of 20 steps at (0.5, 2) on a 10,556-edge graph took 148 us in the pooled kernel, 7 us a step.
+// Draws depend on (walk, step, attempt) alone, so the T lanes of a team evaluate T consecutive attempts at once:
+// all draws, all candidate gathers and all tests of a round are in flight together, and the first accepted attempt
+// (ballot) is the one the serial loop would have stopped at. Attempts behind the first outright acceptance
+// (accept draw below cut2) are never gathered, so the team issues hardly more gathers than the serial loop; what it
+// spends is Philox blocks. T follows the acceptance probability of a try (host side, team_size).
+// Same draws, same decisions, same outputs as the other kernels.
+//
+// The draws of a step's first round are computed under the latency of the row fetch. A step's node stays in the
+// registers of lane (step mod T) and a team writes T consecutive nodes of its row at a time.
+//
+// Requires row descriptors, num_nodes < 2^31 and num_edges < 2^32.
+#pragma once
+#include "walk_kernels.cuh"
+
+namespace walk_b200 {
+
+constexpr int kTeamBlock = 128;
+constexpr int kTeamBlocksPerSm = 10;
+constexpr uint32_t kNoRow = 0xffffffffu;  // a degree: the row is not fetched yet
+
+// GATHER: where a candidate comes from (walk_kernels.cuh). MEMBER: how the membership test is answered.
+template <int T, int MEMBER, int GATHER>
+__global__ void __launch_bounds__(kTeamBlock, kTeamBlocksPerSm) node2vec_team_kernel(const Node2vecParams P) {
+  static_assert(T >= 2 && T <= 32 && (T & (T - 1)) == 0, "whole teams per warp");
+  constexpr unsigned kFull = 0xffffffffu;
+  const int lane = threadIdx.x & 31, sub = lane & (T - 1), base = lane & ~(T - 1);
+  const unsigned team = (T == 32 ? kFull : ((1u << (T & 31)) - 1u)) << base;
+  const unsigned before = (1u << lane) - 1u;
+  const int32_t L = P.walk_length;
+  const int64_t n = P.num_walks;
+  const uint32_t cut01 = max(P.cut0, P.cut1);
+  const StepReader<GATHER> reader(P.col, P.steps, P.step_bits);
+  const L2Policy pol = make_policies(P.hints);
+
+  // Walks are dealt statically when every one has a team of its own (queue == NULL: nothing to clear before the
+  // launch), else taken from the launch-wide counter, as many at a time as the warp has teams.
+  const int64_t warp_id = ((int64_t)blockIdx.x * kTeamBlock + threadIdx.x) >> 5;
+  int64_t q_next = 0, q_end = 0;
+  bool drained = false;
+  if (!P.queue) {
+    q_next = warp_id * (32 / T);
+    q_end = min(q_next + 32 / T, n);
+    drained = true;
+  }
+
+  bool active = false;
+  uint32_t i = 0;                  // walk (row of this launch)
+  int32_t l = 0;
+  uint32_t v = 0, t = 0;           // current and previous node
+  uint32_t rs = 0, deg = kNoRow;   // row of v
+  uint32_t t_rs = 0, t_deg = 0;    // row of t
+  uint32_t buf_x = 0, buf_e = 0;   // this lane's share of the team's unwritten steps (edge + 1, 0: none)
+
+  auto put = [&](int32_t step, int64_t node, int64_t edge) {
+    st8(P.n_out + (int64_t)i * ((int64_t)L + 1) + 1 + step, node, pol.stream);
+    if (P.e_out) st8(P.e_out + (int64_t)i * L + step, edge, pol.stream);
+  };
+
+  auto fetch_row = [&](uint32_t node, uint32_t& start, uint32_t& degree) {
+    const uint64_t d = (uint64_t)ld8(P.desc + node, pol.keep);
+    start = (uint32_t)(d & kDescStartMask);
+    degree = (uint32_t)(d >> kDescStartBits);
+    if ((d & kDescStartMask) + degree > (uint64_t)P.num_edges) {
+      raise_flag(P.flags, WALK_B200_FLAG_BAD_ROWPTR);
+      degree = 0;
+    }
+  };
+
+  while (true) {
+    const unsigned idle = __ballot_sync(kFull, !active);
+    if (idle) {
+      if (q_next >= q_end && !drained) {
+        unsigned long long chunk = 0;
+        if (lane == 0) chunk = atomicAdd(P.queue, 1ull);
+        chunk = __shfl_sync(kFull, chunk, 0);
+        if ((int64_t)chunk * (32 / T) < n) {
+          q_next = (int64_t)chunk * (32 / T);
+          q_end = min(q_next + 32 / T, n);
+        } else {
+          drained = true;
+        }
+      }
+      if (q_next < q_end) {
+        const int64_t mine = q_next + __popc(idle & ((1u << base) - 1u)) / T;
+        if (!active && mine < q_end) {
+          i = (uint32_t)mine;
+          const int64_t first = ld8(P.start + mine, pol.stream);
+          if (sub == 0) st8(P.n_out + mine * ((int64_t)L + 1), first, pol.stream);
+          active = L > 0;
+          if ((uint64_t)first >= (uint64_t)P.num_nodes) {
+            if (sub == 0) raise_flag(P.flags, WALK_B200_FLAG_BAD_NODE);
+            for (int32_t k = sub; k < L; k += T) put(k, first, -1);
+            active = false;
+          }
+          v = (uint32_t)first;
+          t = v;
+          l = 0;
+          deg = kNoRow;
+        }
+        q_next = min(q_end, q_next + __popc(idle) / T);
+      } else if (idle == kFull) {
+        break;
+      }
+    }
+
+    // ---- row of v, and meanwhile the draws of the first round
+    if (active && deg == kNoRow) fetch_row(v, rs, deg);
+    const uint64_t gw = P.walk_index_base + (uint64_t)i * P.walk_index_stride;
+    uint32_t cand, acc;
+    node2vec_draw(P.key0, P.key1, gw, (uint32_t)l, (uint32_t)sub, cand, acc);
+    uint32_t x = v, e = 0;                // the step's node and edge + 1
+    uint32_t x_rs = 0, x_deg = kNoRow;    // row of x where the gather brings it along
+    bool finished = false;
+    if (active && deg == 0) {  // stay in place for every remaining step
+      const int32_t flushed = l & ~(T - 1);
+      if (flushed + sub < l) put(flushed + sub, buf_x, (int64_t)buf_e - 1);
+      for (int32_t k = l + sub; k < L; k += T) put(k, v, -1);
+      finished = true;
+    }
+    const bool stepping = active && !finished;
+    const uint32_t inv = stepping ? 0xffffffffu / deg : 0u;
+    auto slot = [&](uint32_t c) -> uint32_t {  // cand % deg, exactly (see node2vec_walk_kernel)
+      uint32_t rem = c - __umulhi(c, inv) * deg;
+      if (rem >= deg) rem -= deg;
+      return rs + rem;
+    };
+    auto gather = [&](uint32_t edge, uint32_t& to, uint32_t& to_rs, uint32_t& to_deg) {
+      if (!reader.read(edge, pol, (uint64_t)P.num_nodes, to, to_rs, to_deg)) {
+        raise_flag(P.flags, WALK_B200_FLAG_BAD_NODE);
+        to = v;  // park on the current node
+        to_rs = rs; to_deg = deg;
+      }
+    };
+
+    // ---- first step and rows of one entry: no rejection
+    const bool plain = stepping && (l == 0 || deg == 1);
+    const uint32_t cand0 = __shfl_sync(kFull, cand, base);
+    if (plain) {
+      e = slot(cand0);
+      gather(e, x, x_rs, x_deg);
+      e++;
+    }
+    // ---- rounds of T attempts
+    bool searching = stepping && !plain;
+    uint32_t a0 = 0;
+    while (__any_sync(kFull, searching)) {
+      if (a0) node2vec_draw(P.key0, P.key1, gw, (uint32_t)l, a0 + (uint32_t)sub, cand, acc);
+      const bool valid = searching && a0 + (uint32_t)sub < P.max_attempts;
+      const unsigned out = __ballot_sync(kFull, valid && acc < P.cut2) & team;
+      const unsigned upto = out ? (out & (0u - out)) * 2u - 1u : kFull;  // lanes up to the first outright acceptance
+      const bool outright = valid && acc < P.cut2;
+      const bool need = valid && (upto >> lane & 1u) && (outright || acc < cut01);
+      uint32_t c_e = 0, c_x = 0, c_rs = 0, c_deg = kNoRow;
+      if (need) {
+        c_e = slot(cand);
+        gather(c_e, c_x, c_rs, c_deg);
+      }
+      bool ok = need && (outright || (c_x == t && acc < P.cut0));
+      const unsigned known = __ballot_sync(kFull, ok) & team;
+      if (need && !ok && acc < P.cut1 && !(known & before)) {  // nothing before it is accepted yet: ask
+        if (MEMBER == MEMBER_HASH) {
+          ok = edge_lookup(P.edgeset, P.edgeset_buckets, edge_key((uint64_t)c_x, (uint64_t)t));
+        } else if (MEMBER == MEMBER_SEARCH_PREV) {
+          ok = reader.row_contains(t_rs, t_rs + t_deg, c_x, pol);
+        } else {
+          uint32_t s_rs = c_rs, s_deg = c_deg;
+          if (s_deg == kNoRow) fetch_row(c_x, s_rs, s_deg);
+          ok = reader.row_contains(s_rs, s_rs + s_deg, t, pol);
+        }
+      }
+      const unsigned yes = __ballot_sync(kFull, ok) & team;
+      const int win = yes ? __ffs(yes) - 1 : lane;
+      c_x = __shfl_sync(kFull, c_x, win);
+      c_e = __shfl_sync(kFull, c_e, win);
+      if (GATHER == GATHER_PACKED) {
+        c_rs = __shfl_sync(kFull, c_rs, win);
+        c_deg = __shfl_sync(kFull, c_deg, win);
+      }
+      if (searching && yes) {
+        x = c_x; e = c_e + 1; x_rs = c_rs; x_deg = GATHER == GATHER_PACKED ? c_deg : kNoRow;
+        searching = false;
+      }
+      a0 += T;
+      if (searching && a0 >= P.max_attempts) {  // give up on this step: stand still
+        if (sub == 0) raise_flag(P.flags, WALK_B200_FLAG_ATTEMPT_CAP);
+        x_rs = rs; x_deg = deg;
+        searching = false;
+      }
+    }
+    // ---- the step is decided
+    if (stepping) {
+      if ((l & (T - 1)) == sub) { buf_x = x; buf_e = e; }
+      l++;
+      if ((l & (T - 1)) == 0 || l == L) {
+        const int32_t k = ((l - 1) & ~(T - 1)) + sub;
+        if (k < l) put(k, buf_x, (int64_t)buf_e - 1);
+      }
+      t = v; t_rs = rs; t_deg = deg;
+      v = x; rs = x_rs; deg = x_deg;
+      if (l == L) finished = true;
+    }
+    if (finished) active = false;
+  }
+  if (P.queue) finish_queue(P.queue);
+}
+
+}  // namespace walk_b200

@@ -23,6 +23,7 @@
 #include "walk_kernels.cuh"
 #include "n2v_pool.cuh"
 #include "n2v_pool_tri.cuh"
+#include "n2v_team.cuh"
 
 namespace {
 
@@ -72,6 +73,7 @@ struct Tuning {
   std::atomic<int32_t> n2v_rev{1};          // 1 auto (reverse positions when they pay), 0 never, 2 whenever available
   std::atomic<int32_t> n2v_pool{1};         // 1: pooled kernel (walk state in shared memory, one state class per trip)
   std::atomic<int32_t> n2v_blocks_per_sm{0};  // 0 = what the occupancy calculator allows
+  std::atomic<int32_t> n2v_team{0};         // team kernel: 0 where it wins, -1 never, 4/8/16/32 always, with that many lanes
   std::atomic<int32_t> n2v_tri{1};          // 1: use the triangle filter when the graph carries one (undirected graphs), 0 never
   std::atomic<int32_t> n2v_tri_draw_loop{5};  // ... and consume up to this many memory-free rejections per trip there
                                             // (most attempts are: 2 -> 102.9 ms, 3 -> 91.4, 5 -> 87.3, 8 -> 89.5)
@@ -105,6 +107,7 @@ std::atomic<int32_t>* tuning_slot(const char* key) {
   if (!strcmp(key, "n2v_batch_trips")) return &g_tuning.n2v_batch_trips;
   if (!strcmp(key, "n2v_draw_loop")) return &g_tuning.n2v_draw_loop;
   if (!strcmp(key, "n2v_blocks_per_sm")) return &g_tuning.n2v_blocks_per_sm;
+  if (!strcmp(key, "n2v_team")) return &g_tuning.n2v_team;
   if (!strcmp(key, "n2v_tri")) return &g_tuning.n2v_tri;
   if (!strcmp(key, "n2v_tri_draw_loop")) return &g_tuning.n2v_tri_draw_loop;
   if (!strcmp(key, "n2v_count_kernel")) return &g_tuning.n2v_count_kernel;
@@ -141,6 +144,25 @@ int check_walk_sizes(int64_t num_walks, int32_t walk_length, const void* start, 
   if (num_walks > 0 && (int64_t)(walk_length + 1ll) > (INT64_MAX / 8) / num_walks)
     return fail(WALK_B200_ERR_INVALID_ARG, "num_walks * (walk_length + 1) overflows");
   return WALK_B200_OK;
+}
+
+// The graph's step array (see StepReader) if the descriptor carries one.
+int step_array(const walk_b200_csr* g, const void** steps, StepBits* bits) {
+  *steps = nullptr;
+  *bits = StepBits{};
+  if (!(g->flags & WALK_B200_CSR_STEPS)) return WALK_B200_OK;
+  const uint32_t id = g->reserved & 0xffu, start = g->reserved >> 8;
+  if (!g->revpos || (id == 0) != (start == 0) || id > 32 || start > 63)
+    return fail(WALK_B200_ERR_INVALID_ARG, "WALK_B200_CSR_STEPS without a step array from walk_b200_steps_build");
+  *steps = g->revpos;
+  *bits = StepBits{(uint8_t)id, (uint8_t)start};
+  return WALK_B200_OK;
+}
+
+// Gathers of a step array that fits L2 leave their lines there; a larger array streams through.
+int step_hint(const walk_b200_csr* g) {
+  const int64_t bytes = g->num_edges * ((g->flags & WALK_B200_CSR_STEPS) && !g->reserved ? 4 : 8);
+  return bytes <= ((int64_t)128 << 20) ? kHintStepsStay : 0;
 }
 
 int64_t blocks_for(int64_t n) { return (n + kBlock - 1) / kBlock; }
@@ -253,7 +275,7 @@ int sm_count() {
 // kQueueSlots further launches on the same device: more node2vec launches than that in
 // flight at once (across streams) are not supported.
 constexpr int kQueueSlots = 4096;
-__device__ unsigned long long g_queue_slots[kQueueSlots];
+__device__ unsigned long long g_queue_slots[kQueueSlots][2];  // [1]: blocks done, for launches that clear up after themselves
 std::mutex g_queue_mu;
 unsigned long long* g_queue_base[64] = {};
 std::atomic<uint32_t> g_queue_next{0};
@@ -270,7 +292,7 @@ int next_queue_slot(unsigned long long** out) {
       g_queue_base[dev] = static_cast<unsigned long long*>(p);
     }
   }
-  *out = g_queue_base[dev] + (g_queue_next.fetch_add(1) % kQueueSlots);
+  *out = g_queue_base[dev] + 2 * (g_queue_next.fetch_add(1) % kQueueSlots);
   return WALK_B200_OK;
 }
 
@@ -360,11 +382,86 @@ bool tri_applies(const Node2vecParams& P0, int member, bool sym) {
   return pool_possible(P, member) && (g_tuning.n2v_pool.load() == 2 || P.cut1 > P.cut2);
 }
 
+// Lanes per walk of the team kernel, or 0 where another kernel is the better one.
+int team_size(const Node2vecParams& P, int member) {
+  const int mode = g_tuning.n2v_team.load();
+  if (mode < 0 || !P.desc || P.counters || P.num_nodes > 0x7fffffffll || P.num_edges >= 0xffffffffll || P.num_walks >= 0xffffffffll)
+    return 0;
+  if (mode > 0) return mode;
+  // a tuning that asks for one of the other kernels gets it
+  if (g_tuning.n2v_pool.load() != 1 || g_tuning.n2v_rev.load() != 1 || g_tuning.n2v_idx.load() == 1 || g_tuning.n2v_member.load() == 1) return 0;
+  // Measured on R-MAT 17 and 20, 40 steps, against the best other kernel (us; n = walks, 189,440 lanes resident):
+  //   (0.5, 2), hash set:  n = 8,000 T=8 82 of 477 | 32,000 T=4 185 of 519 | 250,000 T=4 648 of 1,029 | 500,000 1,830 of 1,343
+  //   (0.25, 4), hash set: n = 1,000 T=32 61 of 939 | 8,000 T=16 130 of 1,068 | 128,000 T=16 1,089 of 1,520 | 500,000 4,326 of 2,901
+  //   (0.25, 4), search:   n = 500,000 T=16 7,280 of 8,627 | 1,048,576 14,921 of 13,889
+  //   (1, 2), search:      n = 500,000 T=4 1,702 of 2,860 | 1,048,576 4,256 of 4,682
+  // While walks are fewer than the lanes that fit, more lanes per walk cost nothing; beyond that T is about the
+  // number of attempts a step takes (prob_2 bounds it), and from the stated sizes on the serial kernels' better use of
+  // every lane wins -- later for the binary search, whose long chains they cannot overlap.
+  if (P.cut2 >= P.cut0 && P.cut2 >= P.cut1) return 0;  // every first attempt is accepted: nothing to run side by side
+  const bool heavy = P.cut2 < (1u << 28);  // prob_2 below 1/8
+  const int64_t n = P.num_walks, resident = (int64_t)sm_count() * kTeamBlocksPerSm * kTeamBlock;
+  if (n * 32 <= resident) return 32;
+  if (heavy) return n <= (member == MEMBER_HASH ? 200000 : 600000) ? 16 : 0;
+  if (member == MEMBER_HASH && n > 300000) return 0;
+  return n * 12 <= resident ? 8 : 4;
+}
+
+template <int T, int MEMBER, int GATHER>
+int launch_team_k(Node2vecParams P, cudaStream_t s, const char* name) {
+  const auto kernel = node2vec_team_kernel<T, MEMBER, GATHER>;
+  int per_sm = 0;
+  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, kTeamBlock, 0) != cudaSuccess || per_sm <= 0) {
+    (void)cudaGetLastError();
+    per_sm = 4;
+  }
+  const int64_t resident = (int64_t)sm_count() * per_sm;
+  int64_t grid = (P.num_walks * T + kTeamBlock - 1) / kTeamBlock;
+  P.queue = nullptr;
+  if (grid > resident) {
+    grid = resident;
+    if (int rc = next_queue_slot(&P.queue)) return rc;
+  }
+  kernel<<<(unsigned)grid, kTeamBlock, 0, s>>>(P);
+  return check_launch(name);
+}
+
+template <int T, int MEMBER>
+int launch_team_g(const Node2vecParams& P, cudaStream_t s, const char* name) {
+  if (P.steps) {
+    if (P.step_bits.id) return launch_team_k<T, MEMBER, GATHER_PACKED>(P, s, name);
+    return launch_team_k<T, MEMBER, GATHER_COL32>(P, s, name);
+  }
+  return launch_team_k<T, MEMBER, GATHER_COL>(P, s, name);
+}
+
+template <int T>
+int launch_team_t(const Node2vecParams& P, int member, cudaStream_t s, const char* name) {
+  switch (member) {
+    case MEMBER_HASH: return launch_team_g<T, MEMBER_HASH>(P, s, name);
+    case MEMBER_SEARCH_PREV: return launch_team_g<T, MEMBER_SEARCH_PREV>(P, s, name);
+    default: return launch_team_g<T, MEMBER_SEARCH_CAND>(P, s, name);
+  }
+}
+
+int launch_team(const Node2vecParams& P, int lanes, int member, cudaStream_t s, const char* name) {
+  switch (lanes) {
+    case 4: return launch_team_t<4>(P, member, s, name);
+    case 8: return launch_team_t<8>(P, member, s, name);
+    case 16: return launch_team_t<16>(P, member, s, name);
+    default: return launch_team_t<32>(P, member, s, name);
+  }
+}
+
 int launch_n2v(const Node2vecParams& P, bool sym, cudaStream_t s) {
   int member = sym ? MEMBER_SEARCH_PREV : MEMBER_SEARCH_CAND;
   if (P.edgeset && P.edgeset_buckets > 0 && g_tuning.n2v_member.load() != 1) member = MEMBER_HASH;
-  // the triangle filter speaks about "x is a neighbour of t"; the walk asks "t is a neighbour of x": undirected graphs only
-  if (tri_applies(P, member, sym)) {
+  const bool tri = tri_applies(P, member, sym);
+  if (const int lanes = team_size(P, member)) {
+    // reported under the name of the kernel that larger batches of this graph run
+    return launch_team(P, lanes, member, s, tri ? "node2vec_pool_tri_kernel" : pool_applies(P, member) ? "node2vec_pool_kernel" : "node2vec_walk_kernel");
+  }
+  if (tri) {
     Node2vecParams T = P;
     T.draw_loop = g_tuning.n2v_tri_draw_loop.load() < 1 ? 1 : g_tuning.n2v_tri_draw_loop.load();
     if (T.counters) {
@@ -449,6 +546,7 @@ int prepare_n2v(const walk_b200_csr* g, const int64_t* start, int64_t num_walks,
   Node2vecParams P{};
   P.rowptr = g->rowptr; P.col = g->col; P.desc = g->rowdesc;
   P.num_nodes = g->num_nodes; P.num_edges = g->num_edges;
+  if (int rc = step_array(g, &P.steps, &P.step_bits)) return rc;
   P.start = start; P.num_walks = num_walks; P.walk_length = walk_length;
   P.cut0 = cuts[0]; P.cut1 = cuts[1]; P.cut2 = cuts[2];
   P.key0 = (uint32_t)seed; P.key1 = (uint32_t)(seed >> 32);
@@ -466,7 +564,7 @@ int prepare_n2v(const walk_b200_csr* g, const int64_t* start, int64_t num_walks,
   if (P.draw_loop < 1) P.draw_loop = 1;
   P.n_out = n_out; P.e_out = walk_length > 0 ? e_out : nullptr;
   P.flags = status_flags; P.counters = (unsigned long long*)counters;
-  P.hints = g_tuning.l2_hints.load();
+  P.hints = (g_tuning.l2_hints.load() & ~kHintStepsStay) | step_hint(g);
   if (g->edgeset && g->edgeset_buckets > 0) {
     if (g->num_nodes >= 0xffffffffll)
       return fail(WALK_B200_ERR_UNSUPPORTED, "the edge hash set needs num_nodes < 2^32 - 1");

@@ -37,14 +37,16 @@ __device__ __forceinline__ void raise_flag(uint32_t* flags, uint32_t bit) {
 // gathers, rand and the walk matrix stream through once: the former are loaded with an
 // evict-last policy, the latter with evict-first, so that the stream does not flush the
 // row descriptors out of L2. `hints` bit 0 enables the former, bit 1 the latter.
+constexpr int kHintStepsStay = 8;  // set by the launch layer, not by the l2_hints tuning
+
 struct L2Policy {
-  uint64_t keep, stream, normal;
+  uint64_t keep, stream, normal, step;  // step: gathers of the step array (kept like any other line where it can stay in L2)
 };
 
 __device__ __forceinline__ L2Policy make_policies(int hints) {
   L2Policy p;
   if (hints & 4) {  // no explicit policy at all (0 selects the plain load forms below)
-    p.keep = p.stream = p.normal = 0;
+    p.keep = p.stream = p.normal = p.step = 0;
     return p;
   }
   asm("createpolicy.fractional.L2::evict_normal.b64 %0, 1.0;" : "=l"(p.normal));
@@ -52,6 +54,7 @@ __device__ __forceinline__ L2Policy make_policies(int hints) {
   p.stream = p.normal;
   if (hints & 1) asm("createpolicy.fractional.L2::evict_last.b64 %0, 1.0;" : "=l"(p.keep));
   if (hints & 2) asm("createpolicy.fractional.L2::evict_first.b64 %0, 1.0;" : "=l"(p.stream));
+  p.step = (hints & kHintStepsStay) ? p.normal : p.stream;
   return p;
 }
 
@@ -97,6 +100,69 @@ __device__ __forceinline__ void load_row(const int64_t* __restrict__ rowptr,
     deg = b - a;
   }
 }
+
+// ---- step arrays -----------------------------------------------------------------
+// What a step gathers per edge. The walks are bound by random accesses, and the rate of those falls with the size of
+// the array they hit: 2.8e11/s up to 64 MB, 1.04e11 at 128 MB, 6.8e10 at 256 MB, 5.4e10 at 1 GB (gather_probe below).
+// So an edge is gathered from the smallest array that serves the step:
+//   GATHER_COL     the caller's int64 col (8 B per edge; always there)
+//   GATHER_COL32   col as uint32 (4 B per edge)
+//   GATHER_PACKED  8 B per edge: target id | row start << id bits | degree << (id + start bits), where the widths the
+//                  graph needs add up to at most 64. The gather brings the next row along, so a step is one
+//                  dependent access instead of two.
+enum : int { GATHER_COL = 0, GATHER_COL32 = 1, GATHER_PACKED = 2 };
+
+struct StepBits {
+  uint8_t id, start;  // widths of the first two fields of a packed record; 0: no packed records
+};
+
+template <int GATHER>
+struct StepReader {
+  const int64_t* col;
+  const void* steps;
+  uint32_t id_bits, start_bits;
+  __device__ __forceinline__ StepReader(const int64_t* c, const void* s, StepBits b)
+      : col(c), steps(s), id_bits(b.id), start_bits(b.start) {}
+  // Target of an edge and, from packed records, the target's row (row_deg is left alone otherwise). False if the target
+  // is no node of the graph.
+  __device__ __forceinline__ bool read(uint32_t e, const L2Policy& pol, uint64_t num_nodes, uint32_t& to, uint32_t& row_start,
+                                       uint32_t& row_deg) const {
+    if (GATHER == GATHER_COL32) {
+      to = ld4(static_cast<const uint32_t*>(steps) + e, pol.step);
+      return to < num_nodes;
+    }
+    if (GATHER == GATHER_PACKED) {
+      const uint64_t w = (uint64_t)ld8(static_cast<const uint64_t*>(steps) + e, pol.step);
+      to = (uint32_t)(w & ((1ull << id_bits) - 1));
+      row_start = (uint32_t)((w >> id_bits) & ((1ull << start_bits) - 1));
+      row_deg = (uint32_t)(w >> id_bits >> start_bits);
+      return to < num_nodes;
+    }
+    const uint64_t c = (uint64_t)ld8(col + e, pol.step);
+    to = (uint32_t)c;
+    return c < num_nodes;
+  }
+  __device__ __forceinline__ uint32_t id(uint32_t e, const L2Policy& pol) const {
+    if (GATHER == GATHER_COL32) return ld4(static_cast<const uint32_t*>(steps) + e, pol.normal);
+    if (GATHER == GATHER_PACKED) return (uint32_t)((uint64_t)ld8(static_cast<const uint64_t*>(steps) + e, pol.normal) & ((1ull << id_bits) - 1));
+    return (uint32_t)ld8(col + e, pol.normal);
+  }
+  // Is `key` in the ascending row [lo, hi)? Three entries a round, so a round is one memory latency and cuts the row
+  // to a quarter: half the rounds of a binary search for one and a half times its loads.
+  __device__ __forceinline__ bool row_contains(uint32_t lo, uint32_t hi, uint32_t key, const L2Policy& pol) const {
+    while (lo < hi) {
+      const uint32_t q = (hi - lo) >> 2, step = q ? q : 1u;
+      const uint32_t pa = lo + q, pb = min(pa + step, hi - 1), pc = min(pb + step, hi - 1);
+      const uint32_t a = id(pa, pol), b = id(pb, pol), c = id(pc, pol);
+      if (a == key || b == key || c == key) return true;
+      if (key < a) hi = pa;
+      else if (key < b) { lo = pa + 1; hi = pb; }
+      else if (key < c) { lo = pb + 1; hi = pc; }
+      else lo = pc + 1;
+    }
+    return false;
+  }
+};
 
 // ---------------------------------------------------------------------------------
 // gather_probe: what this device sustains in dependent random 8-byte gathers that miss L2.
@@ -594,6 +660,16 @@ __device__ __forceinline__ bool edge_lookup(const uint64_t* __restrict__ table, 
   return true;  // a chain that long does not occur in a table at most half full; "maybe" is the safe answer
 }
 
+// The launch's own chunk counter (queue[0]) goes back to zero for the slot's next user: every block counts itself out in
+// queue[1] when its warps have read the counter for the last time, and the last one clears both.
+__device__ __forceinline__ void finish_queue(unsigned long long* queue) {
+  __syncthreads();
+  if (threadIdx.x == 0 && atomicAdd(queue + 1, 1ull) + 1 == gridDim.x) {
+    queue[0] = 0;
+    queue[1] = 0;
+  }
+}
+
 __global__ void __launch_bounds__(kBlock) trifilter_build_kernel(const int64_t* __restrict__ rowptr,
                                                                  const int64_t* __restrict__ col,
                                                                  const uint64_t* __restrict__ colrev,
@@ -667,6 +743,8 @@ struct Node2vecParams {
   uint64_t edgeset_buckets;
   const uint64_t* colrev;  // REV kernels: col[e] | revpos[e] << 32
   const ulonglong2* colrev16;  // triangle-filter kernel: {colrev[e], filter word of e}
+  const void* steps;       // step array of the graph (see StepReader) or NULL
+  StepBits step_bits;
   int64_t num_nodes, num_edges;
   const int64_t* start;
   int64_t num_walks;

@@ -1,0 +1,62 @@
+"""The team kernel of small node2vec batches: the restatement's walks and edge ids for every team size and membership
+test, at batch sizes around a team, a warp and the launch that starts to use its queue, with step counts around a team's
+write-out, isolated nodes, rows of one entry, self-loops and the attempt cap."""
+import numpy as np
+import pytest
+import torch
+
+import oracle
+from mlx_cluster_b200 import _lib, read_status, rejection_sampling
+from mlx_cluster_b200.ops import WalkGraph
+from tests.test_oracle import random_csr
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(autouse=True)
+def _reset_tuning():
+    yield
+    _lib.set_tuning("n2v_team", 0)
+    _lib.set_tuning("n2v_max_attempts", 1 << 22)
+
+
+@pytest.mark.parametrize("lanes", [0, 4, 8, 16, 32])
+@pytest.mark.parametrize("kind", ["search", "search_prev", "hash"])
+def test_team_walks_are_the_restatements(cuda, lanes, kind):
+    rng = np.random.default_rng(100 + lanes)
+    _lib.set_tuning("n2v_team", lanes)
+    for n_nodes, walks, L, degree in [(40, 1, 1, 3.0), (40, 31, 7, 1.2), (300, 33, 8, 6.0), (300, 257, 33, 40.0),
+                                      (64, 5, 0, 3.0), (2000, 60000, 17, 8.0)]:
+        rowptr, col = random_csr(rng, n_nodes, degree, frac_isolated=0.1, symmetric=kind != "search")
+        start = rng.integers(0, n_nodes, walks).astype(np.int64)
+        graph = WalkGraph(torch.from_numpy(rowptr).to(cuda), torch.from_numpy(col).to(cuda), symmetric=kind == "search_prev",
+                          edgeset=kind == "hash")
+        st = torch.from_numpy(start).to(cuda)
+        for p, q in [(0.25, 4.0), (1.0, 2.0), (0.5, 2.0), (4.0, 0.25)]:
+            want_n, want_e = oracle.node2vec_walk(rowptr, col, start, L, p, q, seed=7, return_edges=True, walk_index_base=3)
+            n, e = rejection_sampling(None, None, st, L, p, q, graph=graph, seed=7, return_edges=True, walk_index_base=3,
+                                      check=True)
+            np.testing.assert_array_equal(n.cpu().numpy(), want_n, err_msg=f"{n_nodes} {walks} {L} {p} {q}")
+            np.testing.assert_array_equal(e.cpu().numpy(), want_e)
+            only = rejection_sampling(None, None, st, L, p, q, graph=graph, seed=7, walk_index_base=3)
+            assert torch.equal(only, n)
+        for cap in (1, 3, 9):  # the cap falls inside and between rounds of a team
+            _lib.set_tuning("n2v_max_attempts", cap)
+            want_n, want_e = oracle.node2vec_walk(rowptr, col, start, L, 0.25, 4.0, seed=7, return_edges=True, max_attempts=cap)
+            n, e = rejection_sampling(None, None, st, L, 0.25, 4.0, graph=graph, seed=7, return_edges=True)
+            np.testing.assert_array_equal(n.cpu().numpy(), want_n)
+            np.testing.assert_array_equal(e.cpu().numpy(), want_e)
+            assert read_status(graph) in (0, _lib.FLAG_ATTEMPT_CAP)
+        _lib.set_tuning("n2v_max_attempts", 1 << 22)
+
+
+def test_team_parks_on_a_bad_start(cuda):
+    rowptr, col = random_csr(np.random.default_rng(5), 50, 4.0, frac_isolated=0.0, symmetric=True)
+    start = np.array([3, 50, -2, 1 << 40, 7], dtype=np.int64)
+    graph = WalkGraph(torch.from_numpy(rowptr).to(cuda), torch.from_numpy(col).to(cuda), symmetric=True)
+    out, e = rejection_sampling(None, None, torch.from_numpy(start).to(cuda), 9, 0.5, 2.0, graph=graph, return_edges=True)
+    assert read_status(graph) == _lib.FLAG_BAD_NODE
+    bad = [1, 2, 3]
+    assert (out.cpu().numpy()[bad] == start[bad][:, None]).all() and (e.cpu().numpy()[bad] == -1).all()
+    want = oracle.node2vec_walk(rowptr, col, start[[0]], 9, 0.5, 2.0, seed=0)
+    np.testing.assert_array_equal(out[[0]].cpu().numpy(), want)
