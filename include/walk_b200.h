@@ -217,6 +217,15 @@ int walk_b200_revpos_build(const walk_b200_csr* g, uint32_t* revpos, uint32_t* s
 int walk_b200_colrev_build(const walk_b200_csr* g, uint64_t* colrev, uint32_t* status_flags, void* stream);
 
 /*
+ * Step array: what a walk step gathers per edge, in the fewest bytes. field_bits = 0: col as uint32, 4 bytes per edge.
+ * Otherwise 8-byte records target | row start << id | degree << (id + start) of the target's row, with
+ * field_bits = id | start << 8; the widths must hold num_nodes and num_edges, and the largest degree must fit the
+ * remaining 64 - id - start bits (the caller's to ensure). num_nodes < 2^31, num_edges < 2^32 - 1. To use it, set
+ * WALK_B200_CSR_STEPS in csr.flags, put the array in csr.revpos and field_bits in csr.reserved; csr.rowdesc must be set.
+ */
+int walk_b200_steps_build(const walk_b200_csr* g, uint32_t field_bits, void* steps, void* stream);
+
+/*
  * Triangle filter for node2vec on an undirected graph: colrev16[e] = {colrev[e], filter word of e} (caller scratch
  * of 16 * num_edges bytes, 16-byte aligned; g needs colrev, edgeset and WALK_B200_CSR_SYMMETRIC). The membership
  * test "is the previous node t a neighbour of the candidate x" (is_neighbor, random_walks/BiasedRandomWalk.cpp:20-28,

@@ -15,7 +15,7 @@ OK = 0
 ERR_INVALID_ARG, ERR_BAD_PQ, ERR_CUDA, ERR_CSR_INVALID, ERR_UNSUPPORTED, ERR_DEVICE_FLAGS = 1, 2, 3, 4, 5, 6
 FLAG_BAD_NODE, FLAG_BAD_EDGE, FLAG_ATTEMPT_CAP, FLAG_BAD_ROWPTR = 0x1, 0x2, 0x4, 0x8
 FLAG_DESC_OVERFLOW, FLAG_UNSORTED_ROW, FLAG_EDGESET_FULL = 0x10, 0x20, 0x80
-CSR_SYMMETRIC, CSR_WANT_EDGESET, CSR_WANT_FUSED, CSR_WANT_TRIFILTER = 0x1, 0x2, 0x4, 0x8
+CSR_SYMMETRIC, CSR_WANT_EDGESET, CSR_WANT_FUSED, CSR_WANT_TRIFILTER, CSR_STEPS = 0x1, 0x2, 0x4, 0x8, 0x10
 COUNTER_NAMES = ("loads", "attempts", "membership", "probes",
                  "steps_deg0", "steps_deg1", "steps_sampled", "steps_first", "formula_probes", "gathers16", "filtered")
 
@@ -24,7 +24,7 @@ EXPORTS = (
     "walk_b200_abi_version", "walk_b200_last_error", "walk_b200_launch_count", "walk_b200_last_kernel",
     "walk_b200_uniform_walk", "walk_b200_uniform_walk_philox", "walk_b200_uniform_draw",
     "walk_b200_uniform_draws", "walk_b200_node2vec_walk", "walk_b200_rowdesc_pack",
-    "walk_b200_csr_validate", "walk_b200_edgeset_buckets", "walk_b200_edgeset_build", "walk_b200_revpos_build", "walk_b200_colrev_build", "walk_b200_trifilter_build", "walk_b200_fused_build", "walk_b200_philox4x32_10", "walk_b200_node2vec_draw",
+    "walk_b200_csr_validate", "walk_b200_edgeset_buckets", "walk_b200_edgeset_build", "walk_b200_revpos_build", "walk_b200_steps_build", "walk_b200_colrev_build", "walk_b200_trifilter_build", "walk_b200_fused_build", "walk_b200_philox4x32_10", "walk_b200_node2vec_draw",
     "walk_b200_node2vec_thresholds", "walk_b200_shard_range", "walk_b200_shard_count_cyclic",
     "walk_b200_graph_create", "walk_b200_graph_destroy", "walk_b200_graph_csr",
     "walk_b200_graph_device_bytes", "walk_b200_uniform_walk_host", "walk_b200_node2vec_walk_host",
@@ -81,6 +81,7 @@ def lib():
     L.walk_b200_edgeset_buckets.argtypes = [i64, C.POINTER(u64)]
     L.walk_b200_edgeset_build.argtypes = [C.POINTER(Csr), vp, u64, vp, vp]
     L.walk_b200_revpos_build.argtypes = [C.POINTER(Csr), vp, vp, vp]
+    L.walk_b200_steps_build.argtypes = [C.POINTER(Csr), C.c_uint32, vp, vp]
     L.walk_b200_colrev_build.argtypes = [C.POINTER(Csr), vp, vp, vp]
     L.walk_b200_trifilter_build.argtypes = [C.POINTER(Csr), vp, i64, vp, vp]
     L.walk_b200_fused_build.argtypes = [C.POINTER(Csr), vp, vp, vp]

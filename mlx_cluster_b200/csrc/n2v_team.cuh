@@ -22,7 +22,6 @@ namespace walk_b200 {
 
 constexpr int kTeamBlock = 128;
 constexpr int kTeamBlocksPerSm = 10;
-constexpr uint32_t kNoRow = 0xffffffffu;  // a degree: the row is not fetched yet
 
 // GATHER: where a candidate comes from (walk_kernels.cuh). MEMBER: how the membership test is answered.
 template <int T, int MEMBER, int GATHER>

@@ -24,6 +24,7 @@
 #include "n2v_pool.cuh"
 #include "n2v_pool_tri.cuh"
 #include "n2v_team.cuh"
+#include "uniform_steps.cuh"
 
 namespace {
 
@@ -251,7 +252,39 @@ int launch_uniform_t(const UniformParams& P, cudaStream_t s) {
   }
 }
 
+template <int SRC, int GATHER, bool HAS_EOUT, int S, int BLOCK, int BLOCKS_PER_SM, bool SECTORS = false>
+int launch_steps_b(const UniformParams& P, cudaStream_t s, const char* name) {
+  const auto kernel = uniform_steps_kernel<SRC, GATHER, HAS_EOUT, S, BLOCK, BLOCKS_PER_SM, SECTORS>;
+  static const cudaError_t carved = cudaFuncSetAttribute(kernel, cudaFuncAttributePreferredSharedMemoryCarveout, 44);  // 100 KB
+  if (carved != cudaSuccess) (void)cudaGetLastError();  // a hint: the launch works without it
+  kernel<<<(unsigned)((P.num_walks + BLOCK - 1) / BLOCK), BLOCK, 0, s>>>(P);
+  return check_launch(name);
+}
+
+// Up to about two generations of walks (300,000) small blocks fill the SMs evenly (200,000 walks, 21 MB graph: 74 us
+// against 88). Beyond, fewer walks in flight with more registers and L1 each are faster: R-MAT 22, every node, 40 steps:
+// 2.77 ms with 1,024 threads per SM, 2.88 with 1,280, 3.02 with 1,536, 3.22 with 2,048. The edge tile doubles the shared
+// memory; at 1,024 threads it takes 3.3 ms against 5.5 with 1,536.
+template <int SRC, int GATHER, bool HAS_EOUT>
+int launch_steps_k(const UniformParams& P, cudaStream_t s, const char* name) {
+  if (P.walk_length <= 8) return launch_steps_b<SRC, GATHER, HAS_EOUT, 8, 64, 16>(P, s, name);
+  if (HAS_EOUT || P.num_walks > 300000) return launch_steps_b<SRC, GATHER, HAS_EOUT, 16, 256, 4, !HAS_EOUT>(P, s, name);
+  return launch_steps_b<SRC, GATHER, HAS_EOUT, 16, 128, SRC == DRAW_NODE2VEC ? 12 : 16>(P, s, name);
+}
+
+template <int SRC>
+int launch_steps(const UniformParams& P, cudaStream_t s, const char* name) {
+  const bool e = P.e_out != nullptr;
+  if (!P.steps) return e ? launch_steps_k<SRC, GATHER_COL, true>(P, s, name) : launch_steps_k<SRC, GATHER_COL, false>(P, s, name);
+  if (P.step_bits.id) return e ? launch_steps_k<SRC, GATHER_PACKED, true>(P, s, name) : launch_steps_k<SRC, GATHER_PACKED, false>(P, s, name);
+  return e ? launch_steps_k<SRC, GATHER_COL32, true>(P, s, name) : launch_steps_k<SRC, GATHER_COL32, false>(P, s, name);
+}
+
 int launch_uniform(const UniformParams& P, cudaStream_t s) {
+  // 16-byte fused records without a step array keep the kernel that reads them
+  if (g_tuning.uniform_variant.load() == 0 && P.desc && P.num_nodes <= 0x7fffffffll && P.num_edges < 0xffffffffll &&
+      !(P.fused && !P.steps && g_tuning.uniform_fused.load() != 0))
+    return P.generate ? launch_steps<DRAW_UNIFORM>(P, s, "uniform_steps_kernel") : launch_steps<DRAW_GIVEN>(P, s, "uniform_steps_kernel");
   const bool d = P.desc != nullptr, e = P.e_out != nullptr;
   if (d) return e ? launch_uniform_t<true, true>(P, s) : launch_uniform_t<true, false>(P, s);
   return e ? launch_uniform_t<false, true>(P, s) : launch_uniform_t<false, false>(P, s);
@@ -382,6 +415,17 @@ bool tri_applies(const Node2vecParams& P0, int member, bool sym) {
   return pool_possible(P, member) && (g_tuning.n2v_pool.load() == 2 || P.cut1 > P.cut2);
 }
 
+// Whether any of the tunings that choose between the node2vec kernels is off its default: who sets them gets what they ask for.
+bool kernel_forced() {
+  return g_tuning.n2v_pool.load() != 1 || g_tuning.n2v_rev.load() != 1 || g_tuning.n2v_idx.load() == 1 || g_tuning.n2v_member.load() == 1;
+}
+
+// Walks that accept by prob_2 alone take uniform steps on the node2vec stream (uniform_steps.cuh).
+bool steps_applies(const Node2vecParams& P) {
+  return P.cut2 >= P.cut0 && P.cut2 >= P.cut1 && P.desc && !P.counters && P.num_nodes <= 0x7fffffffll && P.num_edges < 0xffffffffll &&
+         !kernel_forced();
+}
+
 // Lanes per walk of the team kernel, or 0 where another kernel is the better one.
 int team_size(const Node2vecParams& P, int member) {
   const int mode = g_tuning.n2v_team.load();
@@ -389,7 +433,7 @@ int team_size(const Node2vecParams& P, int member) {
     return 0;
   if (mode > 0) return mode;
   // a tuning that asks for one of the other kernels gets it
-  if (g_tuning.n2v_pool.load() != 1 || g_tuning.n2v_rev.load() != 1 || g_tuning.n2v_idx.load() == 1 || g_tuning.n2v_member.load() == 1) return 0;
+  if (kernel_forced()) return 0;
   // Measured on R-MAT 17 and 20, 40 steps, against the best other kernel (us; n = walks, 189,440 lanes resident):
   //   (0.5, 2), hash set:  n = 8,000 T=8 82 of 477 | 32,000 T=4 185 of 519 | 250,000 T=4 648 of 1,029 | 500,000 1,830 of 1,343
   //   (0.25, 4), hash set: n = 1,000 T=32 61 of 939 | 8,000 T=16 130 of 1,068 | 128,000 T=16 1,089 of 1,520 | 500,000 4,326 of 2,901
@@ -398,7 +442,6 @@ int team_size(const Node2vecParams& P, int member) {
   // While walks are fewer than the lanes that fit, more lanes per walk cost nothing; beyond that T is about the
   // number of attempts a step takes (prob_2 bounds it), and from the stated sizes on the serial kernels' better use of
   // every lane wins -- later for the binary search, whose long chains they cannot overlap.
-  if (P.cut2 >= P.cut0 && P.cut2 >= P.cut1) return 0;  // every first attempt is accepted: nothing to run side by side
   const bool heavy = P.cut2 < (1u << 28);  // prob_2 below 1/8
   const int64_t n = P.num_walks, resident = (int64_t)sm_count() * kTeamBlocksPerSm * kTeamBlock;
   if (n * 32 <= resident) return 32;
@@ -456,6 +499,15 @@ int launch_team(const Node2vecParams& P, int lanes, int member, cudaStream_t s, 
 int launch_n2v(const Node2vecParams& P, bool sym, cudaStream_t s) {
   int member = sym ? MEMBER_SEARCH_PREV : MEMBER_SEARCH_CAND;
   if (P.edgeset && P.edgeset_buckets > 0 && g_tuning.n2v_member.load() != 1) member = MEMBER_HASH;
+  if (steps_applies(P)) {
+    UniformParams U{};
+    U.rowptr = P.rowptr; U.col = P.col; U.desc = P.desc; U.steps = P.steps; U.step_bits = P.step_bits;
+    U.num_nodes = P.num_nodes; U.num_edges = P.num_edges; U.start = P.start; U.num_walks = P.num_walks;
+    U.walk_length = P.walk_length; U.hints = P.hints; U.n_out = P.n_out; U.e_out = P.e_out; U.flags = P.flags;
+    U.key0 = P.key0; U.key1 = P.key1; U.walk_index_base = P.walk_index_base; U.walk_index_stride = P.walk_index_stride;
+    U.cut2 = P.cut2; U.max_attempts = P.max_attempts;
+    return launch_steps<DRAW_NODE2VEC>(U, s, "node2vec_walk_kernel");
+  }
   const bool tri = tri_applies(P, member, sym);
   if (const int lanes = team_size(P, member)) {
     // reported under the name of the kernel that larger batches of this graph run
@@ -753,6 +805,8 @@ int uniform_walk_impl(const walk_b200_csr* g, const int64_t* start, const float*
     P.fused = static_cast<const ulonglong2*>(g->fused);
   }
   P.generate = generate ? 1 : 0;
+  if (int rc = step_array(g, &P.steps, &P.step_bits)) return rc;
+  P.hints = (P.hints & ~kHintStepsStay) | step_hint(g);
   return launch_uniform(P, (cudaStream_t)stream);
 }
 }  // namespace
@@ -815,6 +869,24 @@ int walk_b200_fused_build(const walk_b200_csr* g, void* fused, uint32_t* status_
   fused_build_kernel<<<grid_for_streaming(g->num_edges), kBlock, 0, (cudaStream_t)stream>>>(
       g->col, g->rowdesc, g->num_nodes, g->num_edges, static_cast<ulonglong2*>(fused), status_flags);
   return check_launch("fused_build_kernel");
+}
+
+int walk_b200_steps_build(const walk_b200_csr* g, uint32_t field_bits, void* steps, void* stream) {
+  if (int rc = check_csr(g)) return rc;
+  if (g->num_edges > 0 && !steps) return fail(WALK_B200_ERR_INVALID_ARG, "steps is NULL");
+  if (g->num_nodes > 0x7fffffffll || g->num_edges >= 0xffffffffll)
+    return fail(WALK_B200_ERR_UNSUPPORTED, "step arrays hold 32-bit ids: num_nodes < 2^31 and num_edges < 2^32 - 1");
+  const uint32_t id = field_bits & 0xffu, start = field_bits >> 8;
+  if (field_bits) {
+    if (!g->rowdesc) return fail(WALK_B200_ERR_INVALID_ARG, "packed step records need the row descriptors (rowdesc is NULL)");
+    if (id > 32 || start > 63 || id + start > 63 || (g->num_nodes >> id) != 0 || (g->num_edges >> start) != 0)
+      return fail(WALK_B200_ERR_INVALID_ARG, "field widths %u and %u do not hold %lld nodes and %lld edges", id, start,
+                  (long long)g->num_nodes, (long long)g->num_edges);
+  }
+  if (g->num_edges == 0) return WALK_B200_OK;
+  steps_build_kernel<<<grid_for_streaming(g->num_edges), kBlock, 0, (cudaStream_t)stream>>>(
+      g->col, g->rowdesc, g->num_nodes, g->num_edges, StepBits{(uint8_t)id, (uint8_t)start}, steps);
+  return check_launch("steps_build_kernel");
 }
 
 int walk_b200_colrev_build(const walk_b200_csr* g, uint64_t* colrev, uint32_t* status_flags, void* stream) {
@@ -1137,7 +1209,7 @@ extern "C" int walk_b200_uniform_walk_noalloc(const int64_t* rowptr, const int64
   P.num_nodes = num_nodes; P.num_edges = num_edges;
   P.start = start; P.rand = rand; P.num_walks = num_walks; P.walk_length = walk_length;
   P.n_out = n_out; P.e_out = walk_length > 0 ? e_out : nullptr; P.flags = status_flags;
-  P.hints = g_tuning.l2_hints.load();
+  P.hints = (g_tuning.l2_hints.load() & ~kHintStepsStay) | step_hint(&g);
   return launch_uniform(P, (cudaStream_t)stream);
 }
 

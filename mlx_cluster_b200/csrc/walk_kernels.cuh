@@ -69,8 +69,8 @@ __device__ __forceinline__ int64_t ld8(const void* addr, uint64_t policy) {
 }
 __device__ __forceinline__ uint32_t ld4(const void* addr, uint64_t policy) {
   uint32_t v;
-  if (policy) asm("ld.global.nc.L2::cache_hint.b32 %0, [%1], %2;" : "=r"(v) : "l"(addr), "l"(policy));
-  else asm("ld.global.nc.b32 %0, [%1];" : "=r"(v) : "l"(addr));
+  if (policy) asm("ld.global.nc.L2::cache_hint.L2::64B.b32 %0, [%1], %2;" : "=r"(v) : "l"(addr), "l"(policy));
+  else asm("ld.global.nc.L2::64B.b32 %0, [%1];" : "=r"(v) : "l"(addr));
   return v;
 }
 __device__ __forceinline__ ulonglong2 ld16(const void* addr, uint64_t policy) {
@@ -111,6 +111,8 @@ __device__ __forceinline__ void load_row(const int64_t* __restrict__ rowptr,
 //                  graph needs add up to at most 64. The gather brings the next row along, so a step is one
 //                  dependent access instead of two.
 enum : int { GATHER_COL = 0, GATHER_COL32 = 1, GATHER_PACKED = 2 };
+
+constexpr uint32_t kNoRow = 0xffffffffu;  // a degree: the row is not known yet
 
 struct StepBits {
   uint8_t id, start;  // widths of the first two fields of a packed record; 0: no packed records
@@ -323,6 +325,25 @@ __global__ void __launch_bounds__(kBlock) colrev_build_kernel(const int64_t* __r
   }
 }
 
+// The step array (see StepReader): col as uint32, or with id bits > 0 packed records. An id that is no node becomes the
+// largest value of its field, which the walk flags like the original.
+__global__ void __launch_bounds__(kBlock) steps_build_kernel(const int64_t* __restrict__ col, const uint64_t* __restrict__ desc,
+                                                             int64_t num_nodes, int64_t num_edges, StepBits bits,
+                                                             void* __restrict__ steps) {
+  const int64_t stride = (int64_t)gridDim.x * kBlock;
+  for (int64_t e = (int64_t)blockIdx.x * kBlock + threadIdx.x; e < num_edges; e += stride) {
+    const int64_t c = __ldcs(col + e);
+    const bool node = (uint64_t)c < (uint64_t)num_nodes;
+    if (bits.id == 0) {
+      static_cast<uint32_t*>(steps)[e] = node ? (uint32_t)c : 0xffffffffu;
+    } else {
+      const uint64_t d = node ? __ldg(desc + c) : 0;
+      const uint64_t id = node ? (uint64_t)c : (1ull << bits.id) - 1;
+      static_cast<uint64_t*>(steps)[e] = id | (d & kDescStartMask) << bits.id | (d >> kDescStartBits) << bits.id << bits.start;
+    }
+  }
+}
+
 struct UniformParams {
   const int64_t* rowptr;
   const int64_t* col;
@@ -337,6 +358,9 @@ struct UniformParams {
   int64_t* n_out;
   int64_t* e_out;
   uint32_t* flags;
+  const void* steps;          // step array of the graph (see StepReader) or NULL
+  StepBits step_bits;
+  uint32_t cut2, max_attempts;  // DRAW_NODE2VEC (uniform_steps_kernel)
   int32_t generate;           // draws come from the kernel's own Philox stream instead of `rand`
   uint32_t key0, key1;        // its key
   uint64_t walk_index_base, walk_index_stride;

@@ -99,6 +99,9 @@ class WalkGraph:
         self.colrev = None
         self.colrev16 = None
         self.fused = None
+        self.steps = None         # step array (see build_steps) and the field widths of its records (0: uint32 columns)
+        self.steps_bits = 0
+        self.walk_calls = 0       # walks served: the step array is built on the second
         # size of the edge hash set in 8-byte slots per edge: 2 = half full (the minimum), 4 = a quarter full;
         # None = the library's tuning (default 4), taken when the table fits half of the free device memory
         self.edgeset_slots_per_edge = None if edgeset_slots_per_edge is None else max(2.0, float(edgeset_slots_per_edge))
@@ -106,6 +109,7 @@ class WalkGraph:
             # behind the triangle filter few tests reach the hash set: a sparser table buys nothing there (88.1 against
             # 88.2 ms on the headline workload) and costs its memory
             self.edgeset_slots_per_edge = 2.0
+        self.steps_declined = False
         self.filter_declined = False  # edgeset="auto" looked at this graph for a triangle filter and left it
         self.rows_sorted = None   # None: not checked yet (see check_rows_sorted)
         self.n2v_calls = 0        # node2vec calls served: edgeset="auto" builds the hash set on the second
@@ -135,9 +139,13 @@ class WalkGraph:
                 self.build_trifilter(stream=stream, max_row=trifilter_max_row)
 
     def build_fused(self, stream=None):
-        """Build the fused edge records (16 bytes per edge: target node + its row descriptor) that
-        make a uniform walk step one gather instead of two."""
+        """Build the per-edge records that make a uniform walk step cheap: the step array (:meth:`build_steps`), or for a graph
+        that it cannot hold 16-byte records of the target node and its row descriptor."""
         if self.fused is not None or self.rowdesc is None:
+            return
+        self.build_steps()
+        if self.steps is not None:
+            self.fused = self.steps
             return
         with torch.cuda.device(self.device):
             rec = torch.empty((self.num_edges, 2), dtype=torch.int64, device=self.device)
@@ -148,6 +156,42 @@ class WalkGraph:
             if f:
                 raise ValueError(f"fused record build failed, status flags 0x{f:x}: {describe_flags(f)}")
             self.fused = rec
+
+    def build_steps(self, stream=None):
+        """Build the step array: what a walk gathers per edge, in the fewest bytes (the rate of random accesses falls with the
+        size of the array they hit). While 8 bytes per edge stay within what L2 serves at its full rate, records of the
+        target with its row, so that a step is one dependent access; above that the columns as 4-byte ids."""
+        if self.steps is not None or self.rowdesc is None or self.num_edges == 0:
+            return
+        if self.num_nodes >= 2**31 or self.num_edges >= 2**32 - 1:
+            return
+        with torch.cuda.device(self.device):
+            sh = _stream_handle(stream, self.device)
+            bits = 0
+            if 8 * self.num_edges <= _STEPS_PACKED_BYTES:
+                id_bits, start_bits = self.num_nodes.bit_length(), self.num_edges.bit_length()
+                if id_bits + start_bits + int(self.rowptr.diff().max()).bit_length() <= 64:
+                    bits = id_bits | start_bits << 8
+            steps = torch.empty(self.num_edges, dtype=torch.int64 if bits else torch.int32, device=self.device)
+            csr = self.csr()
+            _lib.check(_lib.lib().walk_b200_steps_build(C.byref(csr), bits, steps.data_ptr(), sh))
+            _sync_stream(stream, self.device)  # a walk on another stream may be the next to read it
+            self.steps, self.steps_bits = steps, bits
+
+    def ready_steps(self, stream=None):
+        """Count a walk and build the step array when the graph turns out to be walked more than once (and there is room for
+        it; never while the stream is being captured)."""
+        self.walk_calls += 1
+        if self.steps is not None or self.walk_calls < 2 or self.rowdesc is None or self.steps_declined:
+            return
+        if torch.cuda.is_current_stream_capturing():
+            return
+        free, _ = torch.cuda.mem_get_info(self.device)
+        cached = torch.cuda.memory_reserved(self.device) - torch.cuda.memory_allocated(self.device)
+        if 8 * self.num_edges > (free + cached) // 4:
+            self.steps_declined = True
+            return
+        self.build_steps(stream=stream)
 
     def build_trifilter(self, stream=None, max_row: Optional[int] = None):
         """Build the triangle filter of an undirected graph (16 bytes per edge; needs ``symmetric=True``, builds the
@@ -211,7 +255,7 @@ class WalkGraph:
                 if self.rows_sorted is None:  # the build checks every row on its way
                     self.rows_sorted = not (f & _lib.FLAG_UNSORTED_ROW)
                 if not f:
-                    csr.revpos = rev.data_ptr()
+                    csr.revpos, csr.flags = rev.data_ptr(), csr.flags & ~_lib.CSR_STEPS
                     joined = torch.empty(self.num_edges, dtype=torch.int64, device=self.device)
                     _lib.check(_lib.lib().walk_b200_colrev_build(C.byref(csr), joined.data_ptr(), self.flags.data_ptr(), sh))
                     f = _take_flags(self.flags, stream, self.device)
@@ -220,10 +264,11 @@ class WalkGraph:
                     self.colrev = joined
 
     def csr(self) -> _lib.Csr:
-        return _lib.Csr(self.rowptr.data_ptr(), _ptr(self.col), self.num_nodes, self.num_edges,
-                        _ptr(self.rowdesc), _lib.CSR_SYMMETRIC if self.symmetric else 0, 0,
-                        _ptr(self.edgeset), self.edgeset_buckets, None, _ptr(self.fused), _ptr(self.colrev),
-                        _ptr(self.colrev16))
+        flags = (_lib.CSR_SYMMETRIC if self.symmetric else 0) | (_lib.CSR_STEPS if self.steps is not None else 0)
+        fused = None if self.fused is self.steps else self.fused
+        return _lib.Csr(self.rowptr.data_ptr(), _ptr(self.col), self.num_nodes, self.num_edges, _ptr(self.rowdesc), flags,
+                        self.steps_bits, _ptr(self.edgeset), self.edgeset_buckets, _ptr(self.steps), _ptr(fused),
+                        _ptr(self.colrev), _ptr(self.colrev16))
 
     def _validate_flags(self, start, check_sorted, stream) -> int:
         with torch.cuda.device(self.device):
@@ -274,6 +319,9 @@ def describe_flags(f: int) -> str:
 _GRAPH_CACHE: "OrderedDict[tuple, WalkGraph]" = OrderedDict()
 _HOST_CACHE: "OrderedDict[tuple, HostGraph]" = OrderedDict()
 _CACHE_SIZE = 4
+# up to here packed step records beat 4-byte columns (200,000 uniform walks: 62 against 67 us on 21 MB of records, 95 against
+# 84 on 58 MB, where the columns still fit L2 whole)
+_STEPS_PACKED_BYTES = 32 << 20
 
 
 def clear_caches() -> None:
@@ -530,6 +578,7 @@ def random_walk(rowptr, col, start, rand, walk_length, *, stream=None, return_ed
             raise ValueError(f"rand must hold n * walk_length = {n * L} values, has {rand.numel()}")
     if validate:
         g.validate(start, check_sorted=False, stream=stream)
+    g.ready_steps(stream)
     with torch.cuda.device(dev):
         if out is None:
             out = torch.empty((n, L + 1), dtype=torch.int64, device=dev)
@@ -675,6 +724,7 @@ def rejection_sampling(rowptr, col, start, walk_length, p, q, *, stream=None, se
     # a graph the caller prepared keeps the structures it was given, except that unsorted rows get the hash set
     _membership_ready(g, edgeset, stream, allow_auto=graph is None, q=q)
     g.n2v_calls += 1
+    g.ready_steps(stream)
     with torch.cuda.device(dev):
         if out is None:
             out = torch.empty((n, L + 1), dtype=torch.int64, device=dev)

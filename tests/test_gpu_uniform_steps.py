@@ -1,0 +1,91 @@
+"""The step-array kernels: uniform walks (draws given, generated, and the node2vec stream of an accept-all (p, q)) over plain
+columns, 4-byte columns and packed records, at walk lengths around a chunk, batch sizes around a warp, a block and the launch
+that writes whole sectors, and outputs that start off a 32-byte boundary. Ids compare exactly with the restatement."""
+import numpy as np
+import pytest
+import torch
+
+import oracle
+from mlx_cluster_b200 import _lib, ops, random_walk, read_status, rejection_sampling
+from mlx_cluster_b200.ops import WalkGraph
+from tests.test_oracle import random_csr
+
+pytestmark = pytest.mark.gpu
+
+GATHERS = ("col", "col32", "packed")
+
+
+def make_graph(dev, rowptr, col, gather, monkeypatch):
+    graph = WalkGraph(torch.from_numpy(rowptr).to(dev), torch.from_numpy(col).to(dev))
+    graph.steps_declined = gather == "col"
+    if gather != "col":
+        monkeypatch.setattr(ops, "_STEPS_PACKED_BYTES", 0 if gather == "col32" else 1 << 40)
+        graph.build_steps()
+        assert (graph.steps_bits != 0) == (gather == "packed") and graph.steps is not None
+    return graph
+
+
+@pytest.mark.parametrize("gather", GATHERS)
+@pytest.mark.parametrize("walks,L", [(1, 1), (31, 8), (33, 9), (64, 16), (65, 17), (300, 80), (300001, 16), (300033, 19)])
+def test_walks_are_the_restatements(cuda, gather, walks, L, monkeypatch):
+    rng = np.random.default_rng(walks + L)
+    rowptr, col = random_csr(rng, 500, 5.0, frac_isolated=0.15, symmetric=bool(L & 1))
+    start = rng.integers(0, 500, walks).astype(np.int64)
+    rand = rng.random((walks, L), dtype=np.float32)
+    graph = make_graph(cuda, rowptr, col, gather, monkeypatch)
+    st, rd = torch.from_numpy(start).to(cuda), torch.from_numpy(rand).to(cuda)
+    n_o, e_o = oracle.uniform_walk(rowptr, col, start, rand, L, return_edges=True)
+    for shift in range(4):  # where the output starts decides which positions end a sector
+        buf = torch.full((walks * (L + 1) + 8,), -7, dtype=torch.int64, device=cuda)
+        out = buf[shift:shift + walks * (L + 1)]
+        random_walk(None, None, st, rd, L, graph=graph, out=out, check=True)
+        np.testing.assert_array_equal(out.cpu().numpy().reshape(walks, L + 1), n_o)
+        assert bool((buf[:shift] == -7).all()) and bool((buf[shift + walks * (L + 1):] == -7).all())
+    n, e = random_walk(None, None, st, rd, L, graph=graph, return_edges=True, check=True)
+    np.testing.assert_array_equal(n.cpu().numpy(), n_o)
+    np.testing.assert_array_equal(e.cpu().numpy(), e_o)
+    n_g, e_g = oracle.uniform_walk(rowptr, col, start, _lib.uniform_draws(5, walks, L, 11, 3), L, return_edges=True)
+    n, e = random_walk(None, None, st, None, L, graph=graph, seed=5, walk_index_base=11, walk_index_stride=3, return_edges=True)
+    np.testing.assert_array_equal(n.cpu().numpy(), n_g)
+    np.testing.assert_array_equal(e.cpu().numpy(), e_g)
+    assert torch.equal(random_walk(None, None, st, None, L, graph=graph, seed=5, walk_index_base=11, walk_index_stride=3), n)
+    for p, q in ((1.0, 1.0), (4.0, 0.25)):
+        n_b, e_b = oracle.node2vec_walk(rowptr, col, start, L, p, q, seed=9, return_edges=True)
+        n, e = rejection_sampling(None, None, st, L, p, q, graph=graph, seed=9, return_edges=True, check=True)
+        np.testing.assert_array_equal(n.cpu().numpy(), n_b)
+        np.testing.assert_array_equal(e.cpu().numpy(), e_b)
+        assert torch.equal(rejection_sampling(None, None, st, L, p, q, graph=graph, seed=9), n)
+
+
+@pytest.mark.parametrize("gather", GATHERS)
+def test_malformed_input_is_flagged(cuda, gather, monkeypatch):
+    """A start that is no node and draws of 1 and NaN stay inside the arrays, as in the other kernels."""
+    rowptr, col = random_csr(np.random.default_rng(2), 100, 4.0, frac_isolated=0.0, symmetric=True)
+    start = np.array([1, 100, -3, 1 << 40, 5, 6], dtype=np.int64)
+    rand = np.full((6, 20), 0.5, dtype=np.float32)
+    rand[4, 3], rand[5, 0] = 1.0, np.nan
+    graph = make_graph(cuda, rowptr, col, gather, monkeypatch)
+    out, e = random_walk(None, None, torch.from_numpy(start).to(cuda), torch.from_numpy(rand).to(cuda), 20, graph=graph,
+                         return_edges=True)
+    assert read_status(graph) & _lib.FLAG_BAD_NODE
+    out, e = out.cpu().numpy(), e.cpu().numpy()
+    assert (out[1:4] == start[1:4, None]).all() and (e[1:4] == -1).all() and (out[[0, 4, 5]] < 100).all()
+    np.testing.assert_array_equal(out[0], oracle.uniform_walk(rowptr, col, start[:1], rand[:1], 20)[0])
+
+
+@pytest.mark.parametrize("gather", ("col32", "packed"))
+def test_team_walks_on_the_step_array(cuda, gather, monkeypatch):
+    rng = np.random.default_rng(3)
+    rowptr, col = random_csr(rng, 400, 9.0, frac_isolated=0.1, symmetric=True)
+    start = rng.integers(0, 400, 3000).astype(np.int64)
+    for kw in (dict(symmetric=False), dict(symmetric=True), dict(edgeset=True)):
+        graph = make_graph(cuda, rowptr, col, gather, monkeypatch)
+        graph.symmetric = kw.get("symmetric", False)
+        if kw.get("edgeset"):
+            graph.build_edgeset()
+        for p, q in ((0.5, 2.0), (0.25, 4.0)):
+            want_n, want_e = oracle.node2vec_walk(rowptr, col, start, 21, p, q, seed=4, return_edges=True)
+            n, e = rejection_sampling(None, None, torch.from_numpy(start).to(cuda), 21, p, q, graph=graph, seed=4,
+                                      return_edges=True, check=True)
+            np.testing.assert_array_equal(n.cpu().numpy(), want_n)
+            np.testing.assert_array_equal(e.cpu().numpy(), want_e)
