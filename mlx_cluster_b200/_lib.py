@@ -118,6 +118,29 @@ def lib():
     return L
 
 
+_native = None
+
+
+def native():
+    """The operators' native call path (csrc/native.cpp), bound to the library's entry points."""
+    global _native
+    if _native is None:
+        import importlib.machinery
+        import importlib.util
+        path = _PKG / "_native.so"
+        if not path.exists():
+            raise RuntimeError(f"{path} is missing: build it with `python -m mlx_cluster_b200.build`")
+        loader = importlib.machinery.ExtensionFileLoader("mlx_cluster_b200._native", str(path))
+        m = importlib.util.module_from_spec(importlib.util.spec_from_file_location("mlx_cluster_b200._native", str(path), loader=loader))
+        loader.exec_module(m)
+        L = lib()
+        m.bind(*(C.cast(f, C.c_void_p).value for f in (L.walk_b200_uniform_walk, L.walk_b200_uniform_walk_philox,
+                                                      L.walk_b200_node2vec_walk, L.walk_b200_context_windows,
+                                                      L.walk_b200_negative_walks)))
+        _native = m
+    return _native
+
+
 def check(rc: int) -> None:
     if rc != OK:
         raise WalkError(rc, lib().walk_b200_last_error().decode("utf-8", "replace"))

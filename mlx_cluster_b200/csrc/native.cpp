@@ -1,0 +1,229 @@
+// The operators' call path on CUDA tensors, native: argument checks, output allocation, stream and launch in one call.
+//
+// A small batch is bound by the host: the Python path (device guard, ctypes structure and call, stream look-up, tensor
+// checks) spent 17 us around a kernel of 5 us. Every function here handles the ordinary call and answers
+// NotImplemented for anything else (other dtypes or devices, wrong sizes, unusual argument types), without side effects;
+// the caller then takes the Python path, which words the errors. An int answer is the C ABI's status code.
+// The C ABI is reached through the addresses that bind() is given, so this module links nothing of the library.
+#include <torch/csrc/autograd/python_variable.h>
+
+#include <ATen/ops/empty.h>
+#include <c10/cuda/CUDAGuard.h>
+#include <c10/cuda/CUDAStream.h>
+
+#include <cstdint>
+
+#include "../../include/walk_b200.h"
+
+namespace {
+
+decltype(&walk_b200_uniform_walk) g_uniform;
+decltype(&walk_b200_uniform_walk_philox) g_philox;
+decltype(&walk_b200_node2vec_walk) g_node2vec;
+decltype(&walk_b200_context_windows) g_windows;
+decltype(&walk_b200_negative_walks) g_negatives;
+
+PyObject* decline() { Py_RETURN_NOTIMPLEMENTED; }
+
+// The tensor behind `o` if it is a contiguous CUDA tensor of this dtype on this device (any device if -1).
+const at::Tensor* tensor(PyObject* o, at::ScalarType type, int device) {
+  if (!THPVariable_CheckExact(o)) return nullptr;
+  const at::Tensor& t = THPVariable_Unpack(o);
+  if (t.scalar_type() != type || !t.is_cuda() || !t.is_contiguous() || (device >= 0 && t.get_device() != device)) return nullptr;
+  return &t;
+}
+
+bool word(PyObject* o, uint64_t* v) {
+  if (!PyLong_CheckExact(o)) return false;
+  *v = PyLong_AsUnsignedLongLongMask(o);
+  if (PyErr_Occurred()) { PyErr_Clear(); return false; }
+  return true;
+}
+
+bool length(PyObject* o, int64_t least, int64_t* v) {
+  if (!PyLong_CheckExact(o)) return false;
+  int overflow = 0;
+  *v = PyLong_AsLongLongAndOverflow(o, &overflow);
+  return !overflow && *v >= least && *v <= 0x7ffffffell;
+}
+
+bool number(PyObject* o, double* v) {
+  if (!PyFloat_CheckExact(o) && !PyLong_CheckExact(o)) return false;
+  *v = PyFloat_AsDouble(o);
+  if (PyErr_Occurred()) { PyErr_Clear(); return false; }
+  return true;
+}
+
+void* address(PyObject* o) { return PyLong_AsVoidPtr(o); }
+
+// Raw handle of the stream argument: None is torch's current stream of the device, an int is the handle itself.
+bool stream_of(PyObject* o, int device, void** s) {
+  if (o == Py_None) {
+    *s = (void*)c10::cuda::getCurrentCUDAStream((c10::DeviceIndex)device).stream();
+    return true;
+  }
+  if (!PyLong_CheckExact(o)) return false;
+  *s = address(o);
+  return true;
+}
+
+// `out` of `count` int64 elements on the device, or a new [rows, cols] matrix where it is None.
+bool output(PyObject* o, int64_t rows, int64_t cols, const at::Tensor& like, int device, at::Tensor* t) {
+  if (o == Py_None) {
+    *t = at::empty({rows, cols}, like.options());
+    return true;
+  }
+  const at::Tensor* given = tensor(o, at::kLong, device);
+  if (!given || given->numel() != rows * cols) return false;
+  *t = *given;
+  return true;
+}
+
+int64_t* data(const at::Tensor& t) { return t.numel() ? t.data_ptr<int64_t>() : nullptr; }
+
+// What a call returns: the status if it failed, else the matrix (and the edge matrix).
+PyObject* answer(int rc, PyObject* out_arg, const at::Tensor& out, bool edges, const at::Tensor& e_out) {
+  if (rc != WALK_B200_OK) return PyLong_FromLong(rc);
+  PyObject* o = out_arg == Py_None ? THPVariable_Wrap(out) : (Py_INCREF(out_arg), out_arg);
+  if (!edges) return o;
+  PyObject* e = THPVariable_Wrap(e_out);
+  PyObject* pair = PyTuple_Pack(2, o, e);
+  Py_DECREF(o);
+  Py_DECREF(e);
+  return pair;
+}
+
+// random_walk(csr, flags, device, start, rand | None, length, seed, base, stride, out | None, edges, stream | None)
+PyObject* random_walk(PyObject*, PyObject* const* a, Py_ssize_t n_args) {
+  HANDLE_TH_ERRORS
+  if (n_args != 12) return decline();
+  const int device = (int)PyLong_AsLong(a[2]);
+  const at::Tensor* start = tensor(a[3], at::kLong, device);
+  int64_t L;
+  uint64_t seed, base, stride;
+  void* s;
+  if (!start || !length(a[5], 0, &L) || !word(a[6], &seed) || !word(a[7], &base) || !word(a[8], &stride) ||
+      !stream_of(a[11], device, &s))
+    return decline();
+  const int64_t n = start->numel();
+  const at::Tensor* rand = nullptr;
+  if (a[4] != Py_None && (!(rand = tensor(a[4], at::kFloat, device)) || rand->numel() != n * L)) return decline();
+  const bool edges = a[10] == Py_True;
+  c10::cuda::CUDAGuard guard((c10::DeviceIndex)device);
+  at::Tensor out, e_out;
+  if (!output(a[9], n, L + 1, *start, device, &out)) return decline();
+  if (edges) e_out = at::empty({n, L}, start->options());
+  const walk_b200_csr* csr = static_cast<const walk_b200_csr*>(address(a[0]));
+  uint32_t* flags = static_cast<uint32_t*>(address(a[1]));
+  int64_t* e = edges ? data(e_out) : nullptr;
+  int rc;
+  Py_BEGIN_ALLOW_THREADS
+  if (rand) rc = g_uniform(csr, data(*start), rand->numel() ? rand->data_ptr<float>() : nullptr, n, (int32_t)L, data(out), e, flags, s);
+  else rc = g_philox(csr, data(*start), n, (int32_t)L, seed, base, stride, data(out), e, flags, s);
+  Py_END_ALLOW_THREADS
+  return answer(rc, a[9], out, edges, e_out);
+  END_HANDLE_TH_ERRORS
+}
+
+// rejection_sampling(csr, flags, device, start, length, p, q, seed, base, stride, out | None, edges, stream | None)
+PyObject* rejection_sampling(PyObject*, PyObject* const* a, Py_ssize_t n_args) {
+  HANDLE_TH_ERRORS
+  if (n_args != 13) return decline();
+  const int device = (int)PyLong_AsLong(a[2]);
+  const at::Tensor* start = tensor(a[3], at::kLong, device);
+  int64_t L;
+  double p, q;
+  uint64_t seed, base, stride;
+  void* s;
+  if (!start || !length(a[4], 0, &L) || !number(a[5], &p) || !number(a[6], &q) || !word(a[7], &seed) || !word(a[8], &base) ||
+      !word(a[9], &stride) || !stream_of(a[12], device, &s))
+    return decline();
+  const int64_t n = start->numel();
+  const bool edges = a[11] == Py_True;
+  c10::cuda::CUDAGuard guard((c10::DeviceIndex)device);
+  at::Tensor out, e_out;
+  if (!output(a[10], n, L + 1, *start, device, &out)) return decline();
+  if (edges) e_out = at::empty({n, L}, start->options());
+  const walk_b200_csr* csr = static_cast<const walk_b200_csr*>(address(a[0]));
+  uint32_t* flags = static_cast<uint32_t*>(address(a[1]));
+  int rc;
+  Py_BEGIN_ALLOW_THREADS
+  rc = g_node2vec(csr, data(*start), n, (int32_t)L, p, q, seed, base, stride, data(out), edges ? data(e_out) : nullptr, flags,
+                  nullptr, s);
+  Py_END_ALLOW_THREADS
+  return answer(rc, a[10], out, edges, e_out);
+  END_HANDLE_TH_ERRORS
+}
+
+// context_windows(walks, context_size, out | None, stream | None)
+PyObject* context_windows(PyObject*, PyObject* const* a, Py_ssize_t n_args) {
+  HANDLE_TH_ERRORS
+  if (n_args != 4) return decline();
+  const at::Tensor* walks = tensor(a[0], at::kLong, -1);
+  int64_t cs;
+  void* s;
+  if (!walks || walks->dim() != 2 || !length(a[1], 1, &cs) || cs > walks->size(1) || walks->size(1) > 0x7fffffffll) return decline();
+  const int device = (int)walks->get_device();
+  if (!stream_of(a[3], device, &s)) return decline();
+  const int64_t n = walks->size(0), row = walks->size(1);
+  c10::cuda::CUDAGuard guard((c10::DeviceIndex)device);
+  at::Tensor out;
+  if (!output(a[2], n * (row + 1 - cs), cs, *walks, device, &out)) return decline();
+  int rc;
+  Py_BEGIN_ALLOW_THREADS
+  rc = g_windows(data(*walks), n, (int32_t)(row - 1), (int32_t)cs, data(out), s);
+  Py_END_ALLOW_THREADS
+  return answer(rc, a[2], out, false, out);
+  END_HANDLE_TH_ERRORS
+}
+
+// negative_walks(start, length, num_nodes, seed, base, stride, out | None, stream | None)
+PyObject* negative_walks(PyObject*, PyObject* const* a, Py_ssize_t n_args) {
+  HANDLE_TH_ERRORS
+  if (n_args != 8) return decline();
+  const at::Tensor* start = tensor(a[0], at::kLong, -1);
+  int64_t L;
+  uint64_t nodes, seed, base, stride;
+  void* s;
+  if (!start || start->dim() != 1 || !length(a[1], 0, &L) || !word(a[2], &nodes) || nodes > (1ull << 32) || !word(a[3], &seed) ||
+      !word(a[4], &base) || !word(a[5], &stride))
+    return decline();
+  const int device = (int)start->get_device();
+  if (!stream_of(a[7], device, &s)) return decline();
+  const int64_t n = start->numel();
+  c10::cuda::CUDAGuard guard((c10::DeviceIndex)device);
+  at::Tensor out;
+  if (!output(a[6], n, L + 1, *start, device, &out)) return decline();
+  int rc;
+  Py_BEGIN_ALLOW_THREADS
+  rc = g_negatives(data(*start), n, (int32_t)L, (int64_t)nodes, seed, base, stride, data(out), s);
+  Py_END_ALLOW_THREADS
+  return answer(rc, a[6], out, false, out);
+  END_HANDLE_TH_ERRORS
+}
+
+// bind(uniform_walk, uniform_walk_philox, node2vec_walk, context_windows, negative_walks): addresses of the C ABI
+PyObject* bind(PyObject*, PyObject* const* a, Py_ssize_t n_args) {
+  if (n_args != 5) return decline();
+  g_uniform = reinterpret_cast<decltype(g_uniform)>(address(a[0]));
+  g_philox = reinterpret_cast<decltype(g_philox)>(address(a[1]));
+  g_node2vec = reinterpret_cast<decltype(g_node2vec)>(address(a[2]));
+  g_windows = reinterpret_cast<decltype(g_windows)>(address(a[3]));
+  g_negatives = reinterpret_cast<decltype(g_negatives)>(address(a[4]));
+  if (PyErr_Occurred()) return nullptr;
+  Py_RETURN_NONE;
+}
+
+PyMethodDef methods[] = {
+    {"bind", (PyCFunction)(void (*)(void))bind, METH_FASTCALL, nullptr},
+    {"random_walk", (PyCFunction)(void (*)(void))random_walk, METH_FASTCALL, nullptr},
+    {"rejection_sampling", (PyCFunction)(void (*)(void))rejection_sampling, METH_FASTCALL, nullptr},
+    {"context_windows", (PyCFunction)(void (*)(void))context_windows, METH_FASTCALL, nullptr},
+    {"negative_walks", (PyCFunction)(void (*)(void))negative_walks, METH_FASTCALL, nullptr},
+    {nullptr, nullptr, 0, nullptr}};
+
+PyModuleDef module = {PyModuleDef_HEAD_INIT, "_native", nullptr, -1, methods, nullptr, nullptr, nullptr, nullptr};
+
+}  // namespace
+
+PyMODINIT_FUNC PyInit__native(void) { return PyModule_Create(&module); }

@@ -453,10 +453,14 @@ int team_size(const Node2vecParams& P, int member) {
 template <int T, int MEMBER, int GATHER>
 int launch_team_k(Node2vecParams P, cudaStream_t s, const char* name) {
   const auto kernel = node2vec_team_kernel<T, MEMBER, GATHER>;
-  int per_sm = 0;
-  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, kTeamBlock, 0) != cudaSuccess || per_sm <= 0) {
-    (void)cudaGetLastError();
-    per_sm = 4;
+  static std::atomic<int> blocks_per_sm{0};  // of this kernel; the library is built for one architecture
+  int per_sm = blocks_per_sm.load(std::memory_order_relaxed);
+  if (per_sm == 0) {
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, kTeamBlock, 0) != cudaSuccess || per_sm <= 0) {
+      (void)cudaGetLastError();
+      per_sm = 4;
+    }
+    blocks_per_sm.store(per_sm, std::memory_order_relaxed);
   }
   const int64_t resident = (int64_t)sm_count() * per_sm;
   int64_t grid = (P.num_walks * T + kTeamBlock - 1) / kTeamBlock;

@@ -90,6 +90,7 @@ class WalkGraph:
         if rowptr.dim() != 1 or rowptr.numel() < 1 or col.dim() != 1:
             raise ValueError("rowptr must be 1-D with num_nodes + 1 entries and col 1-D")
         self.device = dev
+        self.stamp = 0            # when it was last fetched from the cache below
         self.num_nodes = rowptr.numel() - 1
         self.num_edges = col.numel()
         self.symmetric = bool(symmetric)
@@ -263,6 +264,30 @@ class WalkGraph:
                         raise ValueError(f"colrev build failed, status flags 0x{f:x}: {describe_flags(f)}")
                     self.colrev = joined
 
+    _CSR_FIELDS = frozenset(("rowptr", "col", "rowdesc", "symmetric", "edgeset", "edgeset_buckets", "steps", "steps_bits", "fused",
+                             "colrev", "colrev16", "flags"))
+    _call = None
+
+    def __setattr__(self, name, value):
+        object.__setattr__(self, name, value)
+        if name in WalkGraph._CSR_FIELDS:
+            object.__setattr__(self, "_call", None)
+
+    def call(self):
+        """(address of the CSR descriptor, address of the status word, device index) for the native call path; kept until a
+        structure of the graph changes."""
+        c = self._call
+        if c is None:
+            csr = self.csr()
+            c = (C.addressof(csr), self.flags.data_ptr(), self.device.index)
+            object.__setattr__(self, "_keep_csr", csr)
+            object.__setattr__(self, "_call", c)
+        return c
+
+    def steps_settled(self) -> bool:
+        """Whether the next walk has nothing to decide about the step array."""
+        return self.steps is not None or self.steps_declined or self.rowdesc is None
+
     def csr(self) -> _lib.Csr:
         flags = (_lib.CSR_SYMMETRIC if self.symmetric else 0) | (_lib.CSR_STEPS if self.steps is not None else 0)
         fused = None if self.fused is self.steps else self.fused
@@ -326,6 +351,7 @@ _STEPS_PACKED_BYTES = 32 << 20
 
 def clear_caches() -> None:
     _GRAPH_CACHE.clear()
+    _RECENT.clear()
     for g in _HOST_CACHE.values():
         g.close()
     _HOST_CACHE.clear()
@@ -352,10 +378,38 @@ def prepare_graph(rowptr, col, *, symmetric: bool = False, edgeset: bool = False
                       trifilter=trifilter)
         _GRAPH_CACHE[k] = g
         while len(_GRAPH_CACHE) > _CACHE_SIZE:
-            _GRAPH_CACHE.popitem(last=False)
-    else:
-        _GRAPH_CACHE.move_to_end(k)
+            old = min((key for key in _GRAPH_CACHE if key != k), key=lambda key: _GRAPH_CACHE[key].stamp)
+            gone = _GRAPH_CACHE.pop(old)
+            _RECENT[:] = [e for e in _RECENT if e[3] is not gone]
+    _stamp(g)
+    _RECENT[:] = [e for e in _RECENT if not (e[0] is rowptr and e[1] is col and e[2] == symmetric)][:2 * _CACHE_SIZE - 1]
+    _RECENT.insert(0, (rowptr, col, symmetric, g, _identity(rowptr, col)))
     return g
+
+
+# Graphs by the tensor objects they were fetched with: what a loop that walks the same graph finds without building a key.
+_RECENT: list = []
+_CLOCK = 0
+
+
+def _stamp(g: "WalkGraph") -> None:
+    global _CLOCK
+    _CLOCK += 1
+    g.stamp = _CLOCK
+
+
+def _identity(rowptr, col):
+    return rowptr.data_ptr(), rowptr._version, col.data_ptr(), col._version
+
+
+def _recent(rowptr, col, symmetric):
+    for e in _RECENT:
+        if e[0] is rowptr and e[1] is col and e[2] == symmetric:
+            if e[4] != _identity(rowptr, col):
+                return None
+            _stamp(e[3])
+            return e[3]
+    return None
 
 
 class HostGraph:
@@ -446,6 +500,13 @@ def _check_walk_length(walk_length):
     if walk_length < 0 or walk_length > 2**31 - 2:
         raise ValueError("walk_length out of range")
     return int(walk_length)
+
+
+def _checked(res):
+    """The native call's answer, its status code raised."""
+    if res.__class__ is int:
+        _lib.check(res)
+    return res
 
 
 def _finish(graph, out, e_out, check, return_edges, stream=None):
@@ -549,6 +610,13 @@ def random_walk(rowptr, col, start, rand, walk_length, *, stream=None, return_ed
     ``gather=True`` the one matrix on ``start``'s device; one process per GPU goes through
     :func:`mlx_cluster_b200.sharded_walk` instead.
     """
+    if devices is None and not validate and not check:
+        g = graph if graph is not None else _recent(rowptr, col, False)
+        if g is not None and g.steps_settled() and (not fused or graph is not None or g.fused is not None):
+            res = _lib.native().random_walk(*g.call(), start, rand, walk_length, seed, walk_index_base, walk_index_stride, out,
+                                            return_edges, None if stream is None else _stream_handle(stream, g.device))
+            if res is not NotImplemented:
+                return _checked(res)
     L = _check_walk_length(walk_length)
     if not isinstance(start, torch.Tensor) or not start.is_cuda:
         if devices is not None:
@@ -631,6 +699,20 @@ def _membership_ready(g: WalkGraph, edgeset, stream, allow_auto: bool = True, q:
         g.build_edgeset(stream=stream)
 
 
+def _membership_settled(g: WalkGraph, edgeset, prepared: bool, q, symmetric, trifilter) -> bool:
+    """Whether :func:`_membership_ready` would leave this graph as it is (an unusual argument answers no)."""
+    if edgeset is not True and edgeset is not False and edgeset != "auto":
+        return False
+    if trifilter and not prepared and (not symmetric or g.colrev16 is None):
+        return False
+    if g.num_edges == 0:
+        return True
+    if g.edgeset is not None:
+        return (prepared or edgeset != "auto" or g.n2v_calls < _FILTER_AFTER_CALLS or g.colrev16 is not None
+                or g.colrev is None or g.filter_declined or q.__class__ not in (int, float) or not q > 1)
+    return g.rows_sorted is True and (edgeset is False or (prepared and edgeset == "auto"))
+
+
 _FILTER_AFTER_CALLS = 16  # the filter takes about 20 launches' time to build and saves a fifth of every launch after
 
 
@@ -689,6 +771,14 @@ def rejection_sampling(rowptr, col, start, walk_length, p, q, *, stream=None, se
     graphs that are walked many times. ``validate``, ``devices`` and ``gather`` as in :func:`random_walk`.
     Returns int64 ``[n, walk_length + 1]``.
     """
+    if devices is None and not validate and not check and not return_counters:
+        g = graph if graph is not None else _recent(rowptr, col, symmetric)
+        if g is not None and g.steps_settled() and _membership_settled(g, edgeset, graph is not None, q, symmetric, trifilter):
+            res = _lib.native().rejection_sampling(*g.call(), start, walk_length, p, q, seed, walk_index_base, walk_index_stride,
+                                                   out, return_edges, None if stream is None else _stream_handle(stream, g.device))
+            if res is not NotImplemented:
+                g.n2v_calls += 1
+                return _checked(res)
     L = _check_walk_length(walk_length)
     p, q = float(p), float(q)
     if edgeset not in (True, False, "auto"):
@@ -803,6 +893,10 @@ def context_windows(walks: torch.Tensor, context_size: int, *, stream=None, out:
     ``[n * (walk_length + 2 - context_size), context_size]``, column 0 the centre node and the rest
     its skip-gram context -- the input of node2vec's positive-pair loss. Same values as
     ``walks.unfold(1, context_size, 1).reshape(-1, context_size)``, produced by one streaming kernel."""
+    if isinstance(walks, torch.Tensor) and walks.is_cuda:
+        res = _lib.native().context_windows(walks, context_size, out, None if stream is None else _stream_handle(stream, walks.device))
+        if res is not NotImplemented:
+            return _checked(res)
     _require(walks, "walks", torch.int64)
     if not walks.is_cuda or walks.dim() != 2:
         raise ValueError("walks must be a 2-D CUDA tensor [n, walk_length + 1]")
@@ -868,6 +962,11 @@ def negative_walks(start: torch.Tensor, walk_length: int, num_nodes: int, *, see
     the other columns node ids drawn uniformly from ``[0, num_nodes)`` (Philox4x32-10, key = ``seed``,
     indexed by global row and column, so shards of the rows reproduce the unsharded result). Feed it to
     :func:`context_windows` like a walk matrix to get the negative pairs of the skip-gram loss."""
+    if isinstance(start, torch.Tensor) and start.is_cuda:
+        res = _lib.native().negative_walks(start, walk_length, num_nodes, seed, row_index_base, row_index_stride, out,
+                                           None if stream is None else _stream_handle(stream, start.device))
+        if res is not NotImplemented:
+            return _checked(res)
     _require(start, "start", torch.int64)
     if not start.is_cuda or start.dim() != 1:
         raise ValueError("start must be a 1-D CUDA tensor")
