@@ -308,24 +308,39 @@ int sm_count() {
 // kQueueSlots further launches on the same device: more node2vec launches than that in
 // flight at once (across streams) are not supported.
 constexpr int kQueueSlots = 4096;
-__device__ unsigned long long g_queue_slots[kQueueSlots][2];  // [1]: blocks done, for launches that clear up after themselves
+__device__ unsigned long long g_queue_slots[kQueueSlots];
+// Slots of the launches that leave theirs as they found it (finish_queue), chunk counter and blocks done: a ring of its
+// own, because the other launches clear their counter before a launch and leave it where it ended.
+__device__ unsigned long long g_clean_queue_slots[kQueueSlots][2];
 std::mutex g_queue_mu;
-unsigned long long* g_queue_base[64] = {};
-std::atomic<uint32_t> g_queue_next{0};
+unsigned long long *g_queue_base[64] = {}, *g_clean_queue_base[64] = {};
+std::atomic<uint32_t> g_queue_next{0}, g_clean_queue_next{0};
+
+int queue_bases(int* dev) {
+  CUDA_TRY(cudaGetDevice(dev));
+  if (*dev < 0 || *dev >= 64) return fail(WALK_B200_ERR_UNSUPPORTED, "device ordinal %d out of range", *dev);
+  std::lock_guard<std::mutex> lock(g_queue_mu);
+  if (!g_queue_base[*dev]) {
+    void *p = nullptr, *c = nullptr;
+    CUDA_TRY(cudaGetSymbolAddress(&p, g_queue_slots));
+    CUDA_TRY(cudaGetSymbolAddress(&c, g_clean_queue_slots));
+    g_queue_base[*dev] = static_cast<unsigned long long*>(p);
+    g_clean_queue_base[*dev] = static_cast<unsigned long long*>(c);
+  }
+  return WALK_B200_OK;
+}
 
 int next_queue_slot(unsigned long long** out) {
   int dev = 0;
-  CUDA_TRY(cudaGetDevice(&dev));
-  if (dev < 0 || dev >= 64) return fail(WALK_B200_ERR_UNSUPPORTED, "device ordinal %d out of range", dev);
-  {
-    std::lock_guard<std::mutex> lock(g_queue_mu);
-    if (!g_queue_base[dev]) {
-      void* p = nullptr;
-      CUDA_TRY(cudaGetSymbolAddress(&p, g_queue_slots));
-      g_queue_base[dev] = static_cast<unsigned long long*>(p);
-    }
-  }
-  *out = g_queue_base[dev] + 2 * (g_queue_next.fetch_add(1) % kQueueSlots);
+  if (int rc = queue_bases(&dev)) return rc;
+  *out = g_queue_base[dev] + g_queue_next.fetch_add(1) % kQueueSlots;
+  return WALK_B200_OK;
+}
+
+int next_clean_queue_slot(unsigned long long** out) {
+  int dev = 0;
+  if (int rc = queue_bases(&dev)) return rc;
+  *out = g_clean_queue_base[dev] + 2 * (g_clean_queue_next.fetch_add(1) % kQueueSlots);
   return WALK_B200_OK;
 }
 
@@ -467,7 +482,7 @@ int launch_team_k(Node2vecParams P, cudaStream_t s, const char* name) {
   P.queue = nullptr;
   if (grid > resident) {
     grid = resident;
-    if (int rc = next_queue_slot(&P.queue)) return rc;
+    if (int rc = next_clean_queue_slot(&P.queue)) return rc;
   }
   kernel<<<(unsigned)grid, kTeamBlock, 0, s>>>(P);
   return check_launch(name);

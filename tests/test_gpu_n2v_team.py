@@ -60,3 +60,20 @@ def test_team_parks_on_a_bad_start(cuda):
     assert (out.cpu().numpy()[bad] == start[bad][:, None]).all() and (e.cpu().numpy()[bad] == -1).all()
     want = oracle.node2vec_walk(rowptr, col, start[[0]], 9, 0.5, 2.0, seed=0)
     np.testing.assert_array_equal(out[[0]].cpu().numpy(), want)
+
+
+def test_team_queue_starts_clean_after_launches_that_leave_theirs_used(cuda):
+    """More launches of the other kernels than the library has counters, then team launches that take their walks from one."""
+    rowptr, col = random_csr(np.random.default_rng(6), 2000, 8.0, frac_isolated=0.0, symmetric=True)
+    start = np.random.default_rng(7).integers(0, 2000, 60000).astype(np.int64)
+    graph = WalkGraph(torch.from_numpy(rowptr).to(cuda), torch.from_numpy(col).to(cuda), symmetric=True)
+    st = torch.from_numpy(start).to(cuda)
+    want = oracle.node2vec_walk(rowptr, col, start, 3, 0.5, 2.0, seed=7)
+    few, buf = st[:64].contiguous(), torch.empty((64, 4), dtype=torch.int64, device=cuda)
+    _lib.set_tuning("n2v_team", -1)
+    for _ in range(4200):
+        rejection_sampling(None, None, few, 3, 0.5, 2.0, graph=graph, seed=7, out=buf)
+    _lib.set_tuning("n2v_team", 16)
+    for _ in range(3):
+        got = rejection_sampling(None, None, st, 3, 0.5, 2.0, graph=graph, seed=7)
+        np.testing.assert_array_equal(got.cpu().numpy(), want)
