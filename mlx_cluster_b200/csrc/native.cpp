@@ -12,6 +12,7 @@
 #include <c10/cuda/CUDAStream.h>
 
 #include <cstdint>
+#include <cstring>
 
 #include "../../include/walk_b200.h"
 
@@ -56,6 +57,13 @@ bool number(PyObject* o, double* v) {
 
 void* address(PyObject* o) { return PyLong_AsVoidPtr(o); }
 
+// A copy of the descriptor in `o` (a bytes object): the graph may replace its own while the call runs without the GIL.
+bool descriptor(PyObject* o, walk_b200_csr* csr) {
+  if (!PyBytes_CheckExact(o) || PyBytes_GET_SIZE(o) != (Py_ssize_t)sizeof(*csr)) return false;
+  std::memcpy(csr, PyBytes_AS_STRING(o), sizeof(*csr));
+  return true;
+}
+
 // Raw handle of the stream argument: None is torch's current stream of the device, an int is the handle itself.
 bool stream_of(PyObject* o, int device, void** s) {
   if (o == Py_None) {
@@ -93,10 +101,11 @@ PyObject* answer(int rc, PyObject* out_arg, const at::Tensor& out, bool edges, c
   return pair;
 }
 
-// random_walk(csr, flags, device, start, rand | None, length, seed, base, stride, out | None, edges, stream | None)
+// random_walk(csr bytes, flags, device, start, rand | None, length, seed, base, stride, out | None, edges, stream | None)
 PyObject* random_walk(PyObject*, PyObject* const* a, Py_ssize_t n_args) {
   HANDLE_TH_ERRORS
-  if (n_args != 12) return decline();
+  walk_b200_csr csr;
+  if (n_args != 12 || !descriptor(a[0], &csr)) return decline();
   const int device = (int)PyLong_AsLong(a[2]);
   const at::Tensor* start = tensor(a[3], at::kLong, device);
   int64_t L;
@@ -113,22 +122,25 @@ PyObject* random_walk(PyObject*, PyObject* const* a, Py_ssize_t n_args) {
   at::Tensor out, e_out;
   if (!output(a[9], n, L + 1, *start, device, &out)) return decline();
   if (edges) e_out = at::empty({n, L}, start->options());
-  const walk_b200_csr* csr = static_cast<const walk_b200_csr*>(address(a[0]));
+  // every address before the GIL goes: a tensor without storage raises
+  const int64_t* from = data(*start);
+  const float* draws = rand && rand->numel() ? rand->data_ptr<float>() : nullptr;
+  int64_t *to = data(out), *e = edges ? data(e_out) : nullptr;
   uint32_t* flags = static_cast<uint32_t*>(address(a[1]));
-  int64_t* e = edges ? data(e_out) : nullptr;
   int rc;
   Py_BEGIN_ALLOW_THREADS
-  if (rand) rc = g_uniform(csr, data(*start), rand->numel() ? rand->data_ptr<float>() : nullptr, n, (int32_t)L, data(out), e, flags, s);
-  else rc = g_philox(csr, data(*start), n, (int32_t)L, seed, base, stride, data(out), e, flags, s);
+  if (rand) rc = g_uniform(&csr, from, draws, n, (int32_t)L, to, e, flags, s);
+  else rc = g_philox(&csr, from, n, (int32_t)L, seed, base, stride, to, e, flags, s);
   Py_END_ALLOW_THREADS
   return answer(rc, a[9], out, edges, e_out);
   END_HANDLE_TH_ERRORS
 }
 
-// rejection_sampling(csr, flags, device, start, length, p, q, seed, base, stride, out | None, edges, stream | None)
+// rejection_sampling(csr bytes, flags, device, start, length, p, q, seed, base, stride, out | None, edges, stream | None)
 PyObject* rejection_sampling(PyObject*, PyObject* const* a, Py_ssize_t n_args) {
   HANDLE_TH_ERRORS
-  if (n_args != 13) return decline();
+  walk_b200_csr csr;
+  if (n_args != 13 || !descriptor(a[0], &csr)) return decline();
   const int device = (int)PyLong_AsLong(a[2]);
   const at::Tensor* start = tensor(a[3], at::kLong, device);
   int64_t L;
@@ -144,12 +156,12 @@ PyObject* rejection_sampling(PyObject*, PyObject* const* a, Py_ssize_t n_args) {
   at::Tensor out, e_out;
   if (!output(a[10], n, L + 1, *start, device, &out)) return decline();
   if (edges) e_out = at::empty({n, L}, start->options());
-  const walk_b200_csr* csr = static_cast<const walk_b200_csr*>(address(a[0]));
+  const int64_t* from = data(*start);
+  int64_t *to = data(out), *e = edges ? data(e_out) : nullptr;
   uint32_t* flags = static_cast<uint32_t*>(address(a[1]));
   int rc;
   Py_BEGIN_ALLOW_THREADS
-  rc = g_node2vec(csr, data(*start), n, (int32_t)L, p, q, seed, base, stride, data(out), edges ? data(e_out) : nullptr, flags,
-                  nullptr, s);
+  rc = g_node2vec(&csr, from, n, (int32_t)L, p, q, seed, base, stride, to, e, flags, nullptr, s);
   Py_END_ALLOW_THREADS
   return answer(rc, a[10], out, edges, e_out);
   END_HANDLE_TH_ERRORS
@@ -169,9 +181,11 @@ PyObject* context_windows(PyObject*, PyObject* const* a, Py_ssize_t n_args) {
   c10::cuda::CUDAGuard guard((c10::DeviceIndex)device);
   at::Tensor out;
   if (!output(a[2], n * (row + 1 - cs), cs, *walks, device, &out)) return decline();
+  const int64_t* from = data(*walks);
+  int64_t* to = data(out);
   int rc;
   Py_BEGIN_ALLOW_THREADS
-  rc = g_windows(data(*walks), n, (int32_t)(row - 1), (int32_t)cs, data(out), s);
+  rc = g_windows(from, n, (int32_t)(row - 1), (int32_t)cs, to, s);
   Py_END_ALLOW_THREADS
   return answer(rc, a[2], out, false, out);
   END_HANDLE_TH_ERRORS
@@ -194,11 +208,27 @@ PyObject* negative_walks(PyObject*, PyObject* const* a, Py_ssize_t n_args) {
   c10::cuda::CUDAGuard guard((c10::DeviceIndex)device);
   at::Tensor out;
   if (!output(a[6], n, L + 1, *start, device, &out)) return decline();
+  const int64_t* from = data(*start);
+  int64_t* to = data(out);
   int rc;
   Py_BEGIN_ALLOW_THREADS
-  rc = g_negatives(data(*start), n, (int32_t)L, (int64_t)nodes, seed, base, stride, data(out), s);
+  rc = g_negatives(from, n, (int32_t)L, (int64_t)nodes, seed, base, stride, to, s);
   Py_END_ALLOW_THREADS
   return answer(rc, a[6], out, false, out);
+  END_HANDLE_TH_ERRORS
+}
+
+// graph_key(rowptr, col, symmetric): the key under which a graph of these tensors is cached, or None where they are not
+// what a graph is made of (contiguous int64 CUDA tensors of one device).
+PyObject* graph_key(PyObject*, PyObject* const* a, Py_ssize_t n_args) {
+  HANDLE_TH_ERRORS
+  if (n_args != 3) Py_RETURN_NONE;
+  const at::Tensor* rowptr = tensor(a[0], at::kLong, -1);
+  const at::Tensor* col = rowptr ? tensor(a[1], at::kLong, (int)rowptr->get_device()) : nullptr;
+  if (!col || rowptr->is_inference() || col->is_inference()) Py_RETURN_NONE;
+  return Py_BuildValue("(KLLKLLiO)", (unsigned long long)(uintptr_t)rowptr->data_ptr(), (long long)rowptr->numel(),
+                       (long long)rowptr->_version(), (unsigned long long)(uintptr_t)col->data_ptr(), (long long)col->numel(),
+                       (long long)col->_version(), (int)rowptr->get_device(), a[2]);
   END_HANDLE_TH_ERRORS
 }
 
@@ -216,6 +246,7 @@ PyObject* bind(PyObject*, PyObject* const* a, Py_ssize_t n_args) {
 
 PyMethodDef methods[] = {
     {"bind", (PyCFunction)(void (*)(void))bind, METH_FASTCALL, nullptr},
+    {"graph_key", (PyCFunction)(void (*)(void))graph_key, METH_FASTCALL, nullptr},
     {"random_walk", (PyCFunction)(void (*)(void))random_walk, METH_FASTCALL, nullptr},
     {"rejection_sampling", (PyCFunction)(void (*)(void))rejection_sampling, METH_FASTCALL, nullptr},
     {"context_windows", (PyCFunction)(void (*)(void))context_windows, METH_FASTCALL, nullptr},

@@ -45,6 +45,13 @@ def _sync_stream(stream, device) -> None:
         torch.cuda.ExternalStream(int(stream), device=device).synchronize()
 
 
+def _capturing(stream, device) -> bool:
+    if stream is None:
+        return torch.cuda.is_current_stream_capturing()
+    with torch.cuda.stream(stream if isinstance(stream, torch.cuda.Stream) else torch.cuda.ExternalStream(int(stream), device=device)):
+        return torch.cuda.is_current_stream_capturing()
+
+
 def _take_flags(flags: torch.Tensor, stream, device) -> int:
     """Read and clear a status word that kernels on ``stream`` may have written. The read waits for that
     stream first: ``Tensor.item()`` alone only orders itself after torch's *current* stream."""
@@ -90,7 +97,6 @@ class WalkGraph:
         if rowptr.dim() != 1 or rowptr.numel() < 1 or col.dim() != 1:
             raise ValueError("rowptr must be 1-D with num_nodes + 1 entries and col 1-D")
         self.device = dev
-        self.stamp = 0            # when it was last fetched from the cache below
         self.num_nodes = rowptr.numel() - 1
         self.num_edges = col.numel()
         self.symmetric = bool(symmetric)
@@ -177,7 +183,8 @@ class WalkGraph:
             csr = self.csr()
             _lib.check(_lib.lib().walk_b200_steps_build(C.byref(csr), bits, steps.data_ptr(), sh))
             _sync_stream(stream, self.device)  # a walk on another stream may be the next to read it
-            self.steps, self.steps_bits = steps, bits
+            self.steps_bits = bits  # before the array: see csr()
+            self.steps = steps
 
     def ready_steps(self, stream=None):
         """Count a walk and build the step array when the graph turns out to be walked more than once (and there is room for
@@ -185,7 +192,7 @@ class WalkGraph:
         self.walk_calls += 1
         if self.steps is not None or self.walk_calls < 2 or self.rowdesc is None or self.steps_declined:
             return
-        if torch.cuda.is_current_stream_capturing():
+        if _capturing(stream, self.device):
             return
         free, _ = torch.cuda.mem_get_info(self.device)
         cached = torch.cuda.memory_reserved(self.device) - torch.cuda.memory_allocated(self.device)
@@ -245,7 +252,8 @@ class WalkGraph:
             f = _take_flags(self.flags, stream, self.device)
             if f:
                 raise ValueError(f"edge set build failed, status flags 0x{f:x}: {describe_flags(f)}")
-            self.edgeset, self.edgeset_buckets = table, buckets
+            self.edgeset_buckets = buckets
+            self.edgeset = table
             # reverse positions ride along when they can be built (rows strictly ascending, < 2^32 - 2
             # edges); they are joined with col into the one array the kernel gathers candidates from
             if self.num_edges < 2**32 - 2 and self.rowdesc is not None and self.num_nodes < 2**32 - 1:
@@ -274,13 +282,11 @@ class WalkGraph:
             object.__setattr__(self, "_call", None)
 
     def call(self):
-        """(address of the CSR descriptor, address of the status word, device index) for the native call path; kept until a
+        """(the CSR descriptor's bytes, address of the status word, device index) for the native call path; kept until a
         structure of the graph changes."""
         c = self._call
         if c is None:
-            csr = self.csr()
-            c = (C.addressof(csr), self.flags.data_ptr(), self.device.index)
-            object.__setattr__(self, "_keep_csr", csr)
+            c = (bytes(self.csr()), self.flags.data_ptr(), self.device.index)
             object.__setattr__(self, "_call", c)
         return c
 
@@ -289,10 +295,11 @@ class WalkGraph:
         return self.steps is not None or self.steps_declined or self.rowdesc is None
 
     def csr(self) -> _lib.Csr:
-        flags = (_lib.CSR_SYMMETRIC if self.symmetric else 0) | (_lib.CSR_STEPS if self.steps is not None else 0)
-        fused = None if self.fused is self.steps else self.fused
+        steps, edgeset = self.steps, self.edgeset  # read once: another thread may be adding a structure
+        flags = (_lib.CSR_SYMMETRIC if self.symmetric else 0) | (_lib.CSR_STEPS if steps is not None else 0)
+        fused = None if self.fused is steps else self.fused
         return _lib.Csr(self.rowptr.data_ptr(), _ptr(self.col), self.num_nodes, self.num_edges, _ptr(self.rowdesc), flags,
-                        self.steps_bits, _ptr(self.edgeset), self.edgeset_buckets, _ptr(self.steps), _ptr(fused),
+                        self.steps_bits if steps is not None else 0, _ptr(edgeset), self.edgeset_buckets, _ptr(steps), _ptr(fused),
                         _ptr(self.colrev), _ptr(self.colrev16))
 
     def _validate_flags(self, start, check_sorted, stream) -> int:
@@ -351,15 +358,15 @@ _STEPS_PACKED_BYTES = 32 << 20
 
 def clear_caches() -> None:
     _GRAPH_CACHE.clear()
-    _RECENT.clear()
     for g in _HOST_CACHE.values():
         g.close()
     _HOST_CACHE.clear()
 
 
 def _key(rowptr, col, symmetric):
+    # native.graph_key makes the same tuple
     return (rowptr.data_ptr(), rowptr.numel(), rowptr._version, col.data_ptr(), col.numel(), col._version,
-            str(rowptr.device), bool(symmetric))
+            rowptr.get_device(), bool(symmetric))
 
 
 def prepare_graph(rowptr, col, *, symmetric: bool = False, edgeset: bool = False, fused: bool = False,
@@ -378,38 +385,22 @@ def prepare_graph(rowptr, col, *, symmetric: bool = False, edgeset: bool = False
                       trifilter=trifilter)
         _GRAPH_CACHE[k] = g
         while len(_GRAPH_CACHE) > _CACHE_SIZE:
-            old = min((key for key in _GRAPH_CACHE if key != k), key=lambda key: _GRAPH_CACHE[key].stamp)
-            gone = _GRAPH_CACHE.pop(old)
-            _RECENT[:] = [e for e in _RECENT if e[3] is not gone]
-    _stamp(g)
-    _RECENT[:] = [e for e in _RECENT if not (e[0] is rowptr and e[1] is col and e[2] == symmetric)][:2 * _CACHE_SIZE - 1]
-    _RECENT.insert(0, (rowptr, col, symmetric, g, _identity(rowptr, col)))
+            _GRAPH_CACHE.popitem(last=False)
+    else:
+        _GRAPH_CACHE.move_to_end(k)
     return g
 
 
-# Graphs by the tensor objects they were fetched with: what a loop that walks the same graph finds without building a key.
-_RECENT: list = []
-_CLOCK = 0
-
-
-def _stamp(g: "WalkGraph") -> None:
-    global _CLOCK
-    _CLOCK += 1
-    g.stamp = _CLOCK
-
-
-def _identity(rowptr, col):
-    return rowptr.data_ptr(), rowptr._version, col.data_ptr(), col._version
-
-
 def _recent(rowptr, col, symmetric):
-    for e in _RECENT:
-        if e[0] is rowptr and e[1] is col and e[2] == symmetric:
-            if e[4] != _identity(rowptr, col):
-                return None
-            _stamp(e[3])
-            return e[3]
-    return None
+    """The cached graph of these tensors, or None: not cached, or not tensors that the cache takes (``prepare_graph``, which
+    builds or refuses, is next then)."""
+    k = _lib.native().graph_key(rowptr, col, bool(symmetric))
+    if k is None:
+        return None
+    g = _GRAPH_CACHE.get(k)
+    if g is not None:
+        _GRAPH_CACHE.move_to_end(k)
+    return g
 
 
 class HostGraph:
