@@ -661,6 +661,14 @@ int grid_for_streaming(int64_t n) {
   return (int)b;
 }
 
+// Rows of a matrix per block of the tile kernels: what the tile holds, but no fewer blocks than fill the device.
+uint32_t tile_rows(int64_t num_rows, int64_t row_len) {
+  int64_t r = kTileEntries / row_len;
+  const int64_t even = (num_rows + 4 * sm_count() - 1) / (4 * sm_count());
+  if (r > even) r = even;
+  return (uint32_t)(r < 1 ? 1 : r);
+}
+
 }  // namespace
 
 namespace walk_b200 {
@@ -988,14 +996,24 @@ int walk_b200_context_windows(const int64_t* walks, int64_t num_walks, int32_t w
   if (per_walk > 0x7fffffffll) return fail(WALK_B200_ERR_UNSUPPORTED, "one walk yields more than 2^31 window elements");
   if (num_walks == 0) return WALK_B200_OK;
   if (!walks || !windows) return fail(WALK_B200_ERR_INVALID_ARG, "walks or windows is NULL");
+  if ((reinterpret_cast<uintptr_t>(walks) & 7) != 0 || (reinterpret_cast<uintptr_t>(windows) & 7) != 0)
+    return fail(WALK_B200_ERR_INVALID_ARG, "walks and windows must be 8-byte aligned");
+  const int64_t row_len = (int64_t)walk_length + 1;
+  if (row_len <= kTileEntries) {
+    const uint32_t rows = tile_rows(num_walks, row_len);
+    const int64_t blocks = (num_walks + rows - 1) / rows;
+    if (blocks <= 0x7fffffffll) {
+      context_windows_tile_kernel<<<(unsigned)blocks, kBlock, 0, (cudaStream_t)stream>>>(
+          walks, num_walks, (uint32_t)row_len, rows, FastDiv((uint32_t)context_size), FastDiv((uint32_t)nwin), windows);
+      return check_launch("context_windows_kernel");
+    }
+  }
   const int64_t bx = (per_walk + 2 * kBlock - 1) / (2 * kBlock);
   dim3 grid((unsigned)(bx < 64 ? bx : 64), (unsigned)(num_walks < 65535 ? num_walks : 65535), 1);
   // division by context_size as a multiply-high when that is exact for every element index of a walk
   const uint64_t magic = (1ull << 32) / (uint64_t)context_size + 1;
   const bool fast = magic <= 0xffffffffull &&
                     (uint64_t)per_walk * (magic * (uint64_t)context_size - (1ull << 32)) < (1ull << 32);
-  if ((reinterpret_cast<uintptr_t>(walks) & 7) != 0 || (reinterpret_cast<uintptr_t>(windows) & 7) != 0)
-    return fail(WALK_B200_ERR_INVALID_ARG, "walks and windows must be 8-byte aligned");
   // the kernel stores pairs of elements with one 16-byte store where the pair starts on a 16-byte boundary;
   // which pairs do depends on where the caller's matrix starts (a view that begins at an odd element is fine)
   const bool base_aligned = (reinterpret_cast<uintptr_t>(windows) & 15) == 0;
@@ -1018,6 +1036,17 @@ int walk_b200_negative_walks(const int64_t* start, int64_t num_rows, int32_t wal
   if (!start || !out) return fail(WALK_B200_ERR_INVALID_ARG, "start or out is NULL");
   const uint32_t quads = walk_length > 0 ? (uint32_t)((walk_length + 3) / 4) : 1u;
   if (num_rows > INT64_MAX / 8 / ((int64_t)walk_length + 1)) return fail(WALK_B200_ERR_INVALID_ARG, "matrix too large");
+  const int64_t row_len = (int64_t)walk_length + 1;
+  if (row_len <= kTileEntries) {
+    const uint32_t rows = tile_rows(num_rows, row_len);
+    const int64_t tiles = (num_rows + rows - 1) / rows;
+    if (tiles <= 0x7fffffffll) {
+      negative_walks_tile_kernel<<<(unsigned)tiles, kBlock, 0, (cudaStream_t)stream>>>(
+          start, num_rows, (uint32_t)row_len, rows, FastDiv(quads), (uint64_t)num_nodes, (uint32_t)seed, (uint32_t)(seed >> 32),
+          row_index_base, row_index_stride ? row_index_stride : 1, out);
+      return check_launch("negative_walks_kernel");
+    }
+  }
   int64_t blocks = blocks_for(num_rows * (int64_t)quads);
   const int64_t cap = (int64_t)sm_count() * 16;
   if (blocks > cap) blocks = cap;

@@ -99,3 +99,24 @@ def test_negative_windows_pipeline(cuda):
     win = context_windows(neg, 5)
     want = neg.unfold(1, 5, 1).reshape(-1, 5)
     assert torch.equal(win, want)
+
+
+@pytest.mark.parametrize("n,L,cs", [(5, 1022, 7), (5, 1023, 1024), (5, 1023, 512), (4, 1024, 9), (30001, 1, 2), (30001, 2, 1),
+                                    (4099, 40, 10), (3, 0, 1)])
+def test_tiles_at_their_edges(cuda, n, L, cs):
+    """Rows that just fit a tile and just do not, tiles of many rows with a ragged last one, into views at either alignment;
+    negative rows of the same shapes against their host replay. Whole numbers: equal."""
+    from mlx_cluster_b200 import negative_walks
+    walks = torch.from_numpy(np.random.default_rng(L).integers(0, 1 << 40, (n, L + 1)).astype(np.int64)).to(cuda)
+    want = walks.unfold(1, cs, 1).reshape(-1, cs)
+    start = walks[:, 0].contiguous()
+    for off in (0, 1):
+        buf = torch.full((want.numel() + 2,), -9, dtype=torch.int64, device=cuda)
+        got = context_windows(walks, cs, out=buf[off:off + want.numel()])
+        assert torch.equal(got.reshape(-1, cs), want)
+        assert int((buf == -9).sum()) == 2
+        buf = torch.full((walks.numel() + 2,), -9, dtype=torch.int64, device=cuda)
+        neg = negative_walks(start, L, 1000, seed=3, row_index_base=5, out=buf[off:off + walks.numel()]).view(n, L + 1)
+        assert torch.equal(neg[:, 0], start) and int((buf == -9).sum()) == 2
+        for r in {0, n // 2, n - 1}:
+            assert neg[r, 1:].tolist() == [_lib.negative_draw(3, 5 + r, k, 1000) for k in range(L)]
