@@ -661,6 +661,12 @@ int grid_for_streaming(int64_t n) {
   return (int)b;
 }
 
+// One warp per chunk of consecutive edges (kEdgeChunk), as many blocks as are resident at once.
+int grid_for_edge_chunks(int64_t n) {
+  const int64_t b = (n + kEdgeChunk * kWarpsPerBlock - 1) / (kEdgeChunk * kWarpsPerBlock), cap = (int64_t)sm_count() * (2048 / kBlock);
+  return (int)(b < cap ? b : cap);
+}
+
 // Rows of a matrix per block of the tile kernels: what the tile holds, but no fewer blocks than fill the device.
 uint32_t tile_rows(int64_t num_rows, int64_t row_len) {
   int64_t r = kTileEntries / row_len;
@@ -966,7 +972,8 @@ int walk_b200_revpos_build(const walk_b200_csr* g, uint32_t* revpos, uint32_t* s
   if (g->num_edges >= 0xfffffffell)
     return fail(WALK_B200_ERR_UNSUPPORTED, "reverse positions are 32-bit: num_edges must be below 2^32 - 2");
   if (g->num_edges == 0) return WALK_B200_OK;
-  revpos_build_kernel<<<grid_for_streaming(g->num_edges), kBlock, 0, (cudaStream_t)stream>>>(
+  CUDA_TRY(cudaMemsetAsync(revpos, 0xff, (size_t)g->num_edges * sizeof(uint32_t), (cudaStream_t)stream));  // kNoEdge
+  revpos_build_kernel<<<grid_for_edge_chunks(g->num_edges), kBlock, 0, (cudaStream_t)stream>>>(
       g->rowptr, g->col, g->num_nodes, g->num_edges, revpos, status_flags);
   return check_launch("revpos_build_kernel");
 }

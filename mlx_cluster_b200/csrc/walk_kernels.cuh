@@ -590,6 +590,33 @@ __device__ __forceinline__ uint64_t edge_bucket(uint64_t key, uint64_t num_bucke
   return __umul64hi(z, num_buckets);
 }
 
+// ---- source rows of consecutive edges ------------------------------------------------------
+// Last row v of [lo, hi) with rowptr[v] <= e, found by a whole warp: 32 probes a round.
+__device__ __forceinline__ int64_t warp_row_of(const int64_t* __restrict__ rowptr, int64_t lo, int64_t hi, int64_t e) {
+  const int lane = threadIdx.x & 31;
+  while (hi - lo > 1) {  // rowptr[lo] <= e < rowptr[hi]
+    const int64_t step = (hi - lo + 31) >> 5, at = lo + step * lane;
+    const unsigned below = __ballot_sync(0xffffffffu, at < hi && (lane == 0 || __ldg(rowptr + at) <= e));
+    const int64_t last = lo + step * (31 - __clz(below));
+    hi = min(hi, last + step);
+    lo = last;
+  }
+  return lo;
+}
+
+// The same by one thread.
+__device__ __forceinline__ int64_t row_of(const int64_t* __restrict__ rowptr, int64_t lo, int64_t hi, int64_t e) {
+  while (hi - lo > 1) {
+    const int64_t mid = lo + (hi - lo) / 2;
+    if (__ldg(rowptr + mid) <= e) lo = mid; else hi = mid;
+  }
+  return lo;
+}
+
+// Per-edge kernels give a warp kEdgeChunk consecutive edges: two searches by the whole warp bound the rows that the chunk
+// lies in, and a lane then looks its own row up among those few (their bounds stay in L1) instead of among all rows.
+constexpr int kEdgeChunk = 256;
+
 __global__ void __launch_bounds__(kBlock) edgeset_build_kernel(const int64_t* __restrict__ rowptr,
                                                                const int64_t* __restrict__ col,
                                                                int64_t num_nodes, int64_t num_edges,
@@ -631,33 +658,39 @@ __global__ void __launch_bounds__(kBlock) edgeset_build_kernel(const int64_t* __
 constexpr uint32_t kNoEdge = 0xffffffffu;       // the reverse edge does not exist
 constexpr uint32_t kUnknownEdge = 0xfffffffeu;  // not looked up: the shortcut must not be taken
 
+// Every pair (u -> v), (v -> u) is settled once, from the end whose target row is the shorter one (ties: the smaller id):
+// that row is searched and both entries are written. Hubs meet in most edges, so the searched rows are short: R-MAT 20,
+// 31 M edges, 1713 us with every edge searching its target's row (and its own row among all) -> 1120. An edge without a
+// reverse keeps the kNoEdge that the host filled the array with.
 __global__ void __launch_bounds__(kBlock) revpos_build_kernel(const int64_t* __restrict__ rowptr,
                                                               const int64_t* __restrict__ col,
                                                               int64_t num_nodes, int64_t num_edges,
                                                               uint32_t* __restrict__ revpos, uint32_t* flags) {
-  const int64_t stride = (int64_t)gridDim.x * kBlock;
-  for (int64_t e = (int64_t)blockIdx.x * kBlock + threadIdx.x; e < num_edges; e += stride) {
-    int64_t lo = 0, hi = num_nodes;  // source row u of edge e: last u with rowptr[u] <= e
-    while (hi - lo > 1) {
-      const int64_t mid = lo + (hi - lo) / 2;
-      if (__ldg(rowptr + mid) <= e) lo = mid; else hi = mid;
-    }
-    const int64_t u = lo;
-    const int64_t v = __ldg(col + e);
-    uint32_t pos = kNoEdge;
-    if ((uint64_t)v >= (uint64_t)num_nodes) {
-      raise_flag(flags, WALK_B200_FLAG_BAD_NODE);
-    } else {
-      if (e > __ldg(rowptr + u) && __ldg(col + e - 1) >= v) raise_flag(flags, WALK_B200_FLAG_UNSORTED_ROW);
-      int64_t a = __ldg(rowptr + v), b = __ldg(rowptr + v + 1);
+  const int64_t warps = (int64_t)gridDim.x * kWarpsPerBlock;
+  for (int64_t c = (int64_t)blockIdx.x * kWarpsPerBlock + (threadIdx.x >> 5); c * kEdgeChunk < num_edges; c += warps) {
+    const int64_t first = c * kEdgeChunk, end = min(first + kEdgeChunk, num_edges);
+    const int64_t row_lo = warp_row_of(rowptr, 0, num_nodes, first);
+    const int64_t row_hi = warp_row_of(rowptr, row_lo, num_nodes, end - 1) + 1;
+    for (int64_t e = first + (threadIdx.x & 31); e < end; e += 32) {
+      const int64_t v = __ldg(col + e);
+      if ((uint64_t)v >= (uint64_t)num_nodes) { raise_flag(flags, WALK_B200_FLAG_BAD_NODE); continue; }
+      const int64_t u = row_of(rowptr, row_lo, row_hi, e);
+      const int64_t u_rs = __ldg(rowptr + u), du = __ldg(rowptr + u + 1) - u_rs;
+      if (e > u_rs && __ldg(col + e - 1) >= v) raise_flag(flags, WALK_B200_FLAG_UNSORTED_ROW);
+      if (u == v) { revpos[e] = (uint32_t)e; continue; }
+      int64_t a = max(__ldg(rowptr + v), (int64_t)0), b = min(__ldg(rowptr + v + 1), num_edges);
+      if (b - a > du || (b - a == du && v > u)) continue;  // the other end's
       while (a < b) {
         const int64_t mid = a + (b - a) / 2;
         const int64_t w = __ldg(col + mid);
-        if (w == u) { pos = (uint32_t)mid; break; }
+        if (w == u) {
+          revpos[e] = (uint32_t)mid;
+          revpos[mid] = (uint32_t)e;
+          break;
+        }
         if (w < u) a = mid + 1; else b = mid;
       }
     }
-    revpos[e] = pos;
   }
 }
 
