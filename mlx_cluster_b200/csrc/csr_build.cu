@@ -10,9 +10,11 @@
 //   3. fill     every edge takes a slot of its row (atomicSub on the same counters) and stores its
 //               32-bit column there: rows are complete but unordered;
 //   4. sort     each row on its own: up to 64 entries by one warp in registers (bitonic network over
-//               two values per lane), longer rows by one block with a least-significant-digit radix
-//               sort whose warps own contiguous pieces of the row (stable without any cross-warp
-//               ordering inside a pass); duplicates are dropped and the row is compacted in place;
+//               two values per lane), up to 2,048 the same with up to 64 values per lane; longer rows by
+//               one block, through a bitmap of the columns where that fits shared memory, else with a
+//               least-significant-digit radix sort whose warps own contiguous pieces of the row (stable
+//               without any cross-warp ordering inside a pass); duplicates are dropped and the row is
+//               compacted in place;
 //   5. scan     surviving entries per row -> rowptr;
 //   6. emit     rows are copied to their final place as int64.
 // Everything is stream-ordered; nothing is read back to the host. Sorted, duplicate-free rows are
@@ -29,8 +31,11 @@ namespace {
 
 constexpr int kBuildBlock = 256;
 constexpr int kBuildWarps = kBuildBlock / 32;
-constexpr uint32_t kSmallRow = 64;         // rows up to this many raw entries: one warp, registers
-constexpr uint32_t kMediumRow = 2048;      // rows up to this many: one warp, radix sort; longer: one block
+constexpr uint32_t kSmallRow = 64;         // rows up to this many raw entries: one warp, two values per lane
+constexpr uint32_t kMediumRow = 1024;      // ... this many: one warp, up to 32 values per lane
+constexpr uint32_t kWideRow = 2048;        // ... this many: one warp, 64 values per lane; longer: one block
+constexpr int kBitmapBits = 20;            // graphs of up to 2^this nodes sort their long rows by bitmap (128 KB)
+constexpr int kBitmapBlock = 1024;
 constexpr uint32_t kPadKey = 0xffffffffu;  // sorts behind every node id (ids are below 2^31)
 constexpr unsigned kFullMask = 0xffffffffu;
 constexpr int kScanItems = 16;             // items per thread of one scan tile
@@ -45,10 +50,20 @@ __device__ __forceinline__ void raise(uint32_t* flags, uint32_t bit) {
 // turned each counter into its row's end offset (32 bits are enough: there are fewer than 2^32
 // slots), so one atomicSub both claims a slot and says where it is. Afterwards the counters are
 // free for the per-row results of the sort.
+// Both are bound by one random access per entry, and by how evenly the atomics spread over L2: those on one line are served
+// one after another, and hubs tend to have neighbouring ids (R-MAT's line 0 takes 1.6 % of all entries). So while the
+// counters fit L2 node v's counter stands at v times an odd constant modulo a power of two (CounterPlace), which leaves no
+// line hotter than its hottest node. R-MAT 20, 16 M edges in: count 705 -> 288 us, fill 774 -> 500 us; ids without hubs
+// 193 -> 187 and 752 -> 767.
+struct CounterPlace {
+  uint32_t mask;  // 0: in node order
+  __host__ __device__ __forceinline__ uint32_t operator()(uint32_t v) const { return mask ? (v * 0x9E3779B1u) & mask : v; }
+};
+
 template <bool FILL>
 __global__ void __launch_bounds__(kBuildBlock) csr_edges_kernel(const int64_t* __restrict__ src,
                                                                 const int64_t* __restrict__ dst, int64_t m,
-                                                                int64_t num_nodes, uint32_t options,
+                                                                int64_t num_nodes, uint32_t options, CounterPlace place,
                                                                 uint32_t* __restrict__ counters,
                                                                 uint32_t* __restrict__ raw_col,
                                                                 uint32_t* __restrict__ flags) {
@@ -62,12 +77,14 @@ __global__ void __launch_bounds__(kBuildBlock) csr_edges_kernel(const int64_t* _
       continue;  // the edge is left out
     }
     if (drop_self && u == v) continue;
+    uint32_t* cu = counters + place((uint32_t)u);
+    uint32_t* cv = counters + place((uint32_t)v);
     if (!FILL) {
-      atomicAdd(counters + u, 1u);
-      if (sym && u != v) atomicAdd(counters + v, 1u);
+      atomicAdd(cu, 1u);
+      if (sym && u != v) atomicAdd(cv, 1u);
     } else {
-      raw_col[atomicSub(counters + u, 1u) - 1u] = (uint32_t)v;
-      if (sym && u != v) raw_col[atomicSub(counters + v, 1u) - 1u] = (uint32_t)u;
+      raw_col[atomicSub(cu, 1u) - 1u] = (uint32_t)v;
+      if (sym && u != v) raw_col[atomicSub(cv, 1u) - 1u] = (uint32_t)u;
     }
   }
 }
@@ -96,6 +113,7 @@ __device__ __forceinline__ uint64_t block_exclusive_scan(uint64_t x, uint64_t* t
 }
 
 __global__ void __launch_bounds__(kBuildBlock) scan_tile_sums_kernel(const uint32_t* __restrict__ in, int64_t n,
+                                                                     CounterPlace place,
                                                                      uint64_t* __restrict__ tile_sums) {
   __shared__ uint64_t warp_sums[kBuildWarps];
   const int64_t base = (int64_t)blockIdx.x * kScanTile;
@@ -103,7 +121,7 @@ __global__ void __launch_bounds__(kBuildBlock) scan_tile_sums_kernel(const uint3
 #pragma unroll
   for (int j = 0; j < kScanItems; j++) {
     const int64_t i = base + (int64_t)j * kBuildBlock + threadIdx.x;
-    if (i < n) mine += in[i];
+    if (i < n) mine += in[place((uint32_t)i)];
   }
   uint64_t total;
   block_exclusive_scan(mine, &total, warp_sums);
@@ -126,7 +144,7 @@ __global__ void __launch_bounds__(kBuildBlock) scan_tile_offsets_kernel(uint64_t
 
 // ENDS: the count of row i is replaced by the low 32 bits of the row's end offset (the fill's cursor).
 template <bool ENDS>
-__global__ void __launch_bounds__(kBuildBlock) scan_write_kernel(uint32_t* __restrict__ in, int64_t n,
+__global__ void __launch_bounds__(kBuildBlock) scan_write_kernel(uint32_t* __restrict__ in, int64_t n, CounterPlace place,
                                                                  const uint64_t* __restrict__ tile_offsets,
                                                                  int64_t* __restrict__ out /* [n + 1] */) {
   __shared__ uint64_t warp_sums[kBuildWarps];
@@ -135,11 +153,12 @@ __global__ void __launch_bounds__(kBuildBlock) scan_write_kernel(uint32_t* __res
 #pragma unroll 1
   for (int j = 0; j < kScanItems; j++) {
     const int64_t i = base + (int64_t)j * kBuildBlock + threadIdx.x;
-    const uint64_t x = i < n ? in[i] : 0;
+    const uint32_t at = place((uint32_t)i);
+    const uint64_t x = i < n ? in[at] : 0;
     uint64_t total;
     const uint64_t ex = block_exclusive_scan(x, &total, warp_sums);
     if (i < n) out[i] = (int64_t)(carry + ex);
-    if (ENDS && i < n) in[i] = (uint32_t)(carry + ex + x);
+    if (ENDS && i < n) in[at] = (uint32_t)(carry + ex + x);
     if (i == n - 1) out[n] = (int64_t)(carry + ex + x);
     carry += total;
   }
@@ -150,152 +169,247 @@ __device__ __forceinline__ uint32_t cmp_swap(uint32_t v, uint32_t other, bool ke
   return keep_min ? min(v, other) : max(v, other);
 }
 
+// A warp takes 32 consecutive rows: their bounds come in with one load, and the entries of its next row are fetched before
+// the current one is sorted. With one row at a time the chain bounds -> entries -> network -> store was exposed row by row:
+// R-MAT 20, a million rows, 430 us -> 118.
 __global__ void __launch_bounds__(kBuildBlock) csr_sort_small_kernel(const int64_t* __restrict__ raw_rowptr,
                                                                      int64_t num_nodes, uint32_t options,
                                                                      uint32_t* __restrict__ raw_col,
                                                                      uint32_t* __restrict__ kept,
                                                                      uint32_t* __restrict__ medium_rows,
+                                                                     uint32_t* __restrict__ wide_rows,
                                                                      uint32_t* __restrict__ long_rows,
                                                                      unsigned long long* __restrict__ list_counts) {
   const bool dedupe = (options & WALK_B200_BUILD_DEDUPE) != 0;
   const int lane = threadIdx.x & 31;
-  const int64_t warps = (int64_t)gridDim.x * kBuildWarps;
-  for (int64_t r = (int64_t)blockIdx.x * kBuildWarps + (threadIdx.x >> 5); r < num_nodes; r += warps) {
-    const int64_t s = raw_rowptr[r];
-    const uint64_t d = (uint64_t)(raw_rowptr[r + 1] - s);
-    if (d == 0) {
-      if (lane == 0) kept[r] = 0;
-      continue;
-    }
-    if (d > kSmallRow) {  // not this kernel's: append to the list of the kernel that sorts it
-      if (lane == 0) {
-        if (d <= kMediumRow) medium_rows[atomicAdd(list_counts + 0, 1ull)] = (uint32_t)r;
-        else long_rows[atomicAdd(list_counts + 1, 1ull)] = (uint32_t)r;
-      }
-      continue;
-    }
-    uint32_t a = (uint32_t)lane < d ? raw_col[s + lane] : kPadKey;
-    uint32_t b = (uint32_t)lane + 32u < d ? raw_col[s + 32 + lane] : kPadKey;
-    // bitonic network over the 64 values a[0..31], b[0..31] (value index = lane, lane + 32)
-    const int top = d > 32 ? 64 : 32;
-    for (int size = 2; size <= top; size <<= 1) {
-      for (int stride = size >> 1; stride > 0; stride >>= 1) {
-        if (stride == 32) {
-          const uint32_t lo = min(a, b), hi = max(a, b);
-          a = lo; b = hi;
-        } else {
+  const unsigned lt = (1u << lane) - 1u;
+  const int64_t r = ((int64_t)blockIdx.x * kBuildWarps + (threadIdx.x >> 5)) * 32 + lane;  // this lane's row
+  const int64_t my_s = raw_rowptr[min(r, num_nodes)];
+  const uint32_t my_d = (uint32_t)(raw_rowptr[min(r + 1, num_nodes)] - my_s);  // 0 beyond the last row
+  if (my_d > kSmallRow) {  // not this kernel's: append to the list of the kernel that sorts it
+    if (my_d <= kMediumRow) medium_rows[atomicAdd(list_counts + 0, 1ull)] = (uint32_t)r;
+    else if (my_d <= kWideRow) wide_rows[atomicAdd(list_counts + 1, 1ull)] = (uint32_t)r;
+    else long_rows[atomicAdd(list_counts + 2, 1ull)] = (uint32_t)r;
+  }
+  uint32_t my_kept = 0;
+  unsigned todo = __ballot_sync(kFullMask, my_d > 0 && my_d <= kSmallRow);
+  int64_t s_next = 0;
+  uint32_t d_next = 0, a_next = kPadKey, b_next = kPadKey;
+  auto fetch = [&](int k) {
+    s_next = __shfl_sync(kFullMask, my_s, k);
+    d_next = __shfl_sync(kFullMask, my_d, k);
+    a_next = (uint32_t)lane < d_next ? raw_col[s_next + lane] : kPadKey;
+    b_next = (uint32_t)lane + 32u < d_next ? raw_col[s_next + 32 + lane] : kPadKey;
+  };
+  if (todo) fetch(__ffs(todo) - 1);
+  while (todo) {
+    const int k = __ffs(todo) - 1;
+    todo &= todo - 1;
+    const int64_t s = s_next;
+    const uint32_t d = d_next;
+    uint32_t a = a_next, b = b_next;
+    if (todo) fetch(__ffs(todo) - 1);
+    // bitonic network over the 64 values a[0..31], b[0..31] (value index = lane, lane + 32), or over a alone
+    if (d <= 32) {
+#pragma unroll
+      for (int size = 2; size <= 32; size <<= 1) {
+#pragma unroll
+        for (int stride = size >> 1; stride > 0; stride >>= 1) {
           const uint32_t oa = __shfl_xor_sync(kFullMask, a, stride);
-          const uint32_t ob = __shfl_xor_sync(kFullMask, b, stride);
-          const bool lower = (lane & stride) == 0;
-          a = cmp_swap(a, oa, lower == ((lane & size) == 0));
-          b = cmp_swap(b, ob, lower == (((lane + 32) & size) == 0));
+          a = cmp_swap(a, oa, ((lane & stride) == 0) == ((lane & size) == 0));
+        }
+      }
+    } else {
+#pragma unroll
+      for (int size = 2; size <= 64; size <<= 1) {
+#pragma unroll
+        for (int stride = size >> 1; stride > 0; stride >>= 1) {
+          if (stride == 32) {
+            const uint32_t lo = min(a, b), hi = max(a, b);
+            a = lo; b = hi;
+          } else {
+            const uint32_t oa = __shfl_xor_sync(kFullMask, a, stride);
+            const uint32_t ob = __shfl_xor_sync(kFullMask, b, stride);
+            const bool lower = (lane & stride) == 0;
+            a = cmp_swap(a, oa, lower == ((lane & size) == 0));
+            b = cmp_swap(b, ob, lower == (((lane + 32) & size) == 0));
+          }
         }
       }
     }
-    // with top == 32 only `a` was a full ascending run; b is all padding then
-    uint32_t prev_a = __shfl_up_sync(kFullMask, a, 1);
+    const uint32_t prev_a = __shfl_up_sync(kFullMask, a, 1);
     uint32_t prev_b = __shfl_up_sync(kFullMask, b, 1);
     const uint32_t last_a = __shfl_sync(kFullMask, a, 31);
     if (lane == 0) prev_b = last_a;
     const bool keep_a = a != kPadKey && (!dedupe || lane == 0 || a != prev_a);
     const bool keep_b = b != kPadKey && (!dedupe || b != prev_b);
     const unsigned ma = __ballot_sync(kFullMask, keep_a), mb = __ballot_sync(kFullMask, keep_b);
-    const unsigned lt = (1u << lane) - 1u;
-    __syncwarp();
     if (keep_a) raw_col[s + __popc(ma & lt)] = a;
     if (keep_b) raw_col[s + __popc(ma) + __popc(mb & lt)] = b;
-    if (lane == 0) kept[r] = (uint32_t)(__popc(ma) + __popc(mb));
+    if (lane == k) my_kept = (uint32_t)(__popc(ma) + __popc(mb));
+  }
+  if (r < num_nodes && my_d <= kSmallRow) kept[r] = my_kept;
+}
+
+// ---- 4b. rows of 65 .. kWideRow entries: one warp, K values per lane -------------------------------
+// The same network over the 32 K values whose index is 32 k + lane: strides of 32 and more stay in a lane. A radix sort
+// between the row and a twin in global memory wrote every entry three times to a random sector, which bound it: R-MAT 20,
+// 405 us -> 195 + 145 us. Two launches, because the registers of 64 values would cost the shorter rows their occupancy.
+// (recursion: a loop over the stages of 64 values is more than the compiler unrolls, and the values must be registers)
+template <int K, int SIZE, int STRIDE>
+__device__ __forceinline__ void sort_network(uint32_t (&v)[K], int lane) {
+  if constexpr (STRIDE >= 32) {
+#pragma unroll
+    for (int k = 0; k < K; k++) {
+      constexpr int kStep = STRIDE >> 5;
+      if ((k & kStep) == 0) {
+        const uint32_t lo = min(v[k], v[k + kStep]), hi = max(v[k], v[k + kStep]);
+        const bool up = ((32 * k) & SIZE) == 0;
+        v[k] = up ? lo : hi;
+        v[k + kStep] = up ? hi : lo;
+      }
+    }
+  } else {
+    const bool lower = (lane & STRIDE) == 0;
+#pragma unroll
+    for (int k = 0; k < K; k++) {
+      const uint32_t o = __shfl_xor_sync(kFullMask, v[k], STRIDE);
+      v[k] = cmp_swap(v[k], o, lower == (((32 * k + lane) & SIZE) == 0));
+    }
+  }
+  if constexpr (STRIDE > 1) sort_network<K, SIZE, STRIDE / 2>(v, lane);
+  else if constexpr (SIZE < 32 * K) sort_network<K, SIZE * 2, SIZE>(v, lane);
+}
+
+template <int K>
+__device__ __forceinline__ uint32_t sort_row_in_registers(uint32_t* __restrict__ row, uint32_t d, bool dedupe) {
+  const int lane = threadIdx.x & 31;
+  const unsigned lt = (1u << lane) - 1u;
+  uint32_t v[K];
+#pragma unroll
+  for (int k = 0; k < K; k++) v[k] = (uint32_t)(32 * k + lane) < d ? row[32 * k + lane] : kPadKey;
+  sort_network<K, 2, 1>(v, lane);
+  uint32_t written = 0, last = 0;
+#pragma unroll
+  for (int k = 0; k < K; k++) {
+    uint32_t prev = __shfl_up_sync(kFullMask, v[k], 1);
+    if (lane == 0) prev = last;
+    last = __shfl_sync(kFullMask, v[k], 31);
+    const bool keep = v[k] != kPadKey && (!dedupe || (k == 0 && lane == 0) || v[k] != prev);
+    const unsigned m = __ballot_sync(kFullMask, keep);
+    if (keep) row[written + (uint32_t)__popc(m & lt)] = v[k];
+    written += (uint32_t)__popc(m);
+  }
+  return written;
+}
+
+template <bool WIDE>
+__global__ void __launch_bounds__(kBuildBlock) csr_sort_listed_kernel(const int64_t* __restrict__ raw_rowptr,
+                                                                      uint32_t options, uint32_t* __restrict__ raw_col,
+                                                                      uint32_t* __restrict__ kept,
+                                                                      const uint32_t* __restrict__ listed,
+                                                                      const unsigned long long* __restrict__ count) {
+  static_assert(kMediumRow == 32 * 32 && kWideRow == 32 * 64, "the limits below");
+  const bool dedupe = (options & WALK_B200_BUILD_DEDUPE) != 0;
+  const unsigned long long rows = *count;
+  const unsigned long long warps = (unsigned long long)gridDim.x * kBuildWarps;
+  for (unsigned long long w = (unsigned long long)blockIdx.x * kBuildWarps + (threadIdx.x >> 5); w < rows; w += warps) {
+    const uint32_t r = listed[w];
+    const int64_t s = raw_rowptr[r];
+    const uint32_t d = (uint32_t)(raw_rowptr[r + 1] - s);
+    uint32_t* row = raw_col + s;
+    uint32_t n;
+    if constexpr (WIDE) {
+      n = sort_row_in_registers<64>(row, d, dedupe);
+    } else {
+      if (d <= 128) n = sort_row_in_registers<4>(row, d, dedupe);
+      else if (d <= 256) n = sort_row_in_registers<8>(row, d, dedupe);
+      else if (d <= 512) n = sort_row_in_registers<16>(row, d, dedupe);
+      else n = sort_row_in_registers<32>(row, d, dedupe);
+    }
+    if ((threadIdx.x & 31) == 0) kept[r] = n;
   }
 }
 
-// ---- 4b. rows of 65 .. kMediumRow entries: one warp, LSD radix sort between the row and its twin ----
-// Same passes as the block kernel below with a team of one warp: no block barrier anywhere, a
-// 256-bin histogram per warp, lane l owns bins 8l .. 8l+7 in the scan.
-__global__ void __launch_bounds__(kBuildBlock) csr_sort_medium_kernel(const int64_t* __restrict__ raw_rowptr,
-                                                                      uint32_t options, int32_t passes, int32_t digit_bits,
-                                                                      uint32_t* __restrict__ raw_col,
-                                                                      uint32_t* __restrict__ tmp,
-                                                                      uint32_t* __restrict__ kept,
-                                                                      const uint32_t* __restrict__ medium_rows,
-                                                                      const unsigned long long* __restrict__ medium_count) {
-  __shared__ uint32_t hist[kBuildWarps][256];
-  const bool dedupe = (options & WALK_B200_BUILD_DEDUPE) != 0;
+// ---- 4c. longer rows, graphs of up to 2^kBitmapBits nodes: a bitmap in shared memory ----------------
+// One block per row. Every entry sets its column's bit, and the set bits in order are the row, sorted and without repeats:
+// the entries are read once and written once. The bitmap is cleared for the next row as it is written out.
+// R-MAT 20 (rows of more than 2,048 entries): 750 us by the radix sort below -> 210 us. With more columns than one bitmap
+// holds, the passes over it cost more than the radix sort (R-MAT 24: 57 ms for the whole build against 51).
+__global__ void __launch_bounds__(kBitmapBlock) csr_bitmap_long_kernel(const int64_t* __restrict__ raw_rowptr,
+                                                                       uint32_t* __restrict__ raw_col,
+                                                                       uint32_t* __restrict__ kept,
+                                                                       const uint32_t* __restrict__ long_rows,
+                                                                       const unsigned long long* __restrict__ long_count) {
+  extern __shared__ uint4 bitmap4[];
+  constexpr int kWarps = kBitmapBlock / 32;
+  constexpr int kGroups = (1 << (kBitmapBits - 7)) / kBitmapBlock;  // 16-byte words of the bitmap per thread
+  static_assert(kWarps == 32, "one lane per warp's sum");
+  __shared__ uint32_t warp_sums[kWarps];
+  uint32_t* bitmap = reinterpret_cast<uint32_t*>(bitmap4);
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const unsigned lt = (1u << lane) - 1u;
-  const uint32_t digit_mask = (1u << digit_bits) - 1u;
-  uint32_t* bins = hist[warp];
-  const unsigned long long rows = *medium_count;
-  const unsigned long long warps = (unsigned long long)gridDim.x * kBuildWarps;
-  for (unsigned long long w = (unsigned long long)blockIdx.x * kBuildWarps + warp; w < rows; w += warps) {
-    const uint32_t r = medium_rows[w];
+  uint4* mine = bitmap4 + warp * 32 * kGroups + lane;  // warp w: a contiguous piece, 32 words of 16 bytes at a time
+#pragma unroll
+  for (int g = 0; g < kGroups; g++) mine[32 * g] = make_uint4(0, 0, 0, 0);
+  __syncthreads();
+  const unsigned long long rows = *long_count;
+  for (unsigned long long w = blockIdx.x; w < rows; w += gridDim.x) {
+    const uint32_t r = long_rows[w];
     const int64_t s = raw_rowptr[r];
     const uint32_t d = (uint32_t)(raw_rowptr[r + 1] - s);
-    uint32_t* cur = raw_col + s;
-    uint32_t* alt = tmp + s;
-    for (int32_t pass = 0; pass < passes; pass++) {
-      const int shift = pass * digit_bits;
+    uint32_t* row = raw_col + s;
+#pragma unroll 4
+    for (uint32_t i = threadIdx.x; i < d; i += kBitmapBlock) {
+      const uint32_t c = row[i], bit = 1u << (c & 31);
+      if (!(bitmap[c >> 5] & bit)) atomicOr(bitmap + (c >> 5), bit);
+    }
+    __syncthreads();
+    uint32_t bits = 0;
 #pragma unroll
-      for (int k = 0; k < 8; k++) bins[lane + 32 * k] = 0;
-      __syncwarp();
-      for (uint32_t i = lane; i < d; i += 32) atomicAdd(&bins[(cur[i] >> shift) & digit_mask], 1u);
-      __syncwarp();
-      {  // exclusive scan of the 256 bins
-        uint32_t c[8], sum = 0;
+    for (int g = 0; g < kGroups; g++) {
+      const uint4 b = mine[32 * g];
+      bits += (uint32_t)(__popc(b.x) + __popc(b.y) + __popc(b.z) + __popc(b.w));
+    }
 #pragma unroll
-        for (int k = 0; k < 8; k++) { c[k] = bins[lane * 8 + k]; sum += c[k]; }
-        uint32_t inc = sum;
+    for (int o = 16; o > 0; o >>= 1) bits += __shfl_xor_sync(kFullMask, bits, o);
+    if (lane == 0) warp_sums[warp] = bits;
+    __syncthreads();
+    const uint32_t sum = warp_sums[lane];
+    uint32_t upto = sum;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const uint32_t y = __shfl_up_sync(kFullMask, upto, o);
+      if (lane >= o) upto += y;
+    }
+    uint32_t before = __shfl_sync(kFullMask, upto - sum, warp);
+    if (threadIdx.x == 31) kept[r] = upto;
+    if (bits) {
+      for (int g = 0; g < kGroups; g++) {
+        const uint4 b = mine[32 * g];
+        const uint32_t own = (uint32_t)(__popc(b.x) + __popc(b.y) + __popc(b.z) + __popc(b.w));
+        if (!__any_sync(kFullMask, own != 0)) continue;
+        uint32_t inc = own;
 #pragma unroll
         for (int o = 1; o < 32; o <<= 1) {
           const uint32_t y = __shfl_up_sync(kFullMask, inc, o);
           if (lane >= o) inc += y;
         }
-        uint32_t run = inc - sum;
+        mine[32 * g] = make_uint4(0, 0, 0, 0);
+        uint32_t at = before + inc - own;
+        const uint32_t word[4] = {b.x, b.y, b.z, b.w};
 #pragma unroll
-        for (int k = 0; k < 8; k++) { bins[lane * 8 + k] = run; run += c[k]; }
-      }
-      __syncwarp();
-      uint32_t v_next = lane < d ? cur[lane] : 0u;
-      for (uint32_t i0 = 0; i0 < d; i0 += 32) {
-        const uint32_t i = i0 + lane;
-        const bool valid = i < d;
-        const uint32_t v = v_next;
-        if (i + 32 < d) v_next = cur[i + 32];
-        const uint32_t digit = valid ? ((v >> shift) & digit_mask) : 0xffffffffu;
-        const unsigned same = __match_any_sync(kFullMask, digit);
-        const uint32_t rank = (uint32_t)__popc(same & lt);
-        uint32_t base = 0;
-        if (valid) base = bins[digit];
-        __syncwarp();
-        if (valid) {
-          alt[base + rank] = v;
-          if (rank == 0) bins[digit] = base + (uint32_t)__popc(same);
+        for (int k = 0; k < 4; k++) {
+          const uint32_t first = ((uint32_t)((warp * kGroups + g) * 32 + lane) * 4 + k) << 5;
+          for (uint32_t left = word[k]; left; left &= left - 1) row[at++] = first + (uint32_t)__ffs(left) - 1u;
         }
-        __syncwarp();
+        before += __shfl_sync(kFullMask, inc, 31);
       }
-      uint32_t* t = cur; cur = alt; alt = t;
     }
-    // drop duplicates, compact to the front of the row in raw_col (in place when cur is the row:
-    // a survivor never moves up, and a step's reads come before its writes)
-    uint32_t* out = raw_col + s;
-    uint32_t written = 0;
-    for (uint32_t i0 = 0; i0 < d; i0 += 32) {
-      const uint32_t i = i0 + lane;
-      uint32_t v = 0;
-      bool keep = false;
-      if (i < d) {
-        v = cur[i];
-        keep = !dedupe || i == 0 || cur[i - 1] != v;
-      }
-      const unsigned m = __ballot_sync(kFullMask, keep);
-      if (keep) out[written + (uint32_t)__popc(m & lt)] = v;
-      written += (uint32_t)__popc(m);
-      __syncwarp();
-    }
-    if (lane == 0) kept[r] = written;
+    __syncthreads();  // every warp has read warp_sums, and its piece of the bitmap is clear
   }
 }
 
-// ---- 4c. longer rows: one block, LSD radix sort between the row and its twin in `tmp` -------------
+// ---- 4d. long rows of larger graphs, or with repeats kept: one block, LSD radix sort between the row and its twin in `tmp` -------------
 // Warp w owns the contiguous piece [w * piece, (w + 1) * piece) of the row. A pass counts digits per
 // warp, turns the counts into one start offset per (digit, warp) -- all of digit k before digit k+1,
 // within a digit warp 0's entries before warp 1's -- and then every warp scatters its piece in order,
@@ -400,40 +514,77 @@ __global__ void __launch_bounds__(kBuildBlock) csr_sort_long_kernel(const int64_
 }
 
 // ---- 6. emit ---------------------------------------------------------------------------------------
+// A warp takes 32 consecutive rows (their bounds in four loads) and has the entries of four of them in flight at a time;
+// the rows on the lists go to a warp (up to kMediumRow entries) or a block each.
+// Streaming: R-MAT 20, 126 MB in and 251 MB out, 230 us with one row at a time -> 138 in all.
 __global__ void __launch_bounds__(kBuildBlock) csr_emit_small_kernel(const int64_t* __restrict__ raw_rowptr,
                                                                      const uint32_t* __restrict__ raw_col,
                                                                      const int64_t* __restrict__ rowptr,
                                                                      int64_t num_nodes, int64_t* __restrict__ col) {
+  constexpr int kAtOnce = 4;
   const int lane = threadIdx.x & 31;
-  const int64_t warps = (int64_t)gridDim.x * kBuildWarps;
-  for (int64_t r = (int64_t)blockIdx.x * kBuildWarps + (threadIdx.x >> 5); r < num_nodes; r += warps) {
-    const int64_t s = raw_rowptr[r];
-    if ((uint64_t)(raw_rowptr[r + 1] - s) > kMediumRow) continue;  // a long row: the block kernel's
-    const int64_t o = rowptr[r];
-    const int64_t k = rowptr[r + 1] - o;
-    for (int64_t j = lane; j < k; j += 32) col[o + j] = (int64_t)raw_col[s + j];
+  const int64_t r = ((int64_t)blockIdx.x * kBuildWarps + (threadIdx.x >> 5)) * 32 + lane;  // this lane's row
+  const int64_t at = min(r, num_nodes), behind = min(r + 1, num_nodes);
+  const int64_t my_s = raw_rowptr[at], my_o = rowptr[at];
+  uint32_t my_k = (uint32_t)(rowptr[behind] - my_o);
+  if ((uint64_t)(raw_rowptr[behind] - my_s) > kSmallRow) my_k = 0;
+#pragma unroll 1
+  for (int k0 = 0; k0 < 32; k0 += kAtOnce) {
+    int64_t s[kAtOnce], o[kAtOnce];
+    uint32_t k[kAtOnce], v[kAtOnce], v2[kAtOnce];
+#pragma unroll
+    for (int j = 0; j < kAtOnce; j++) {
+      s[j] = __shfl_sync(kFullMask, my_s, k0 + j) + lane;
+      o[j] = __shfl_sync(kFullMask, my_o, k0 + j) + lane;
+      k[j] = __shfl_sync(kFullMask, my_k, k0 + j);
+      v[j] = (uint32_t)lane < k[j] ? raw_col[s[j]] : 0u;
+      v2[j] = (uint32_t)lane + 32u < k[j] ? raw_col[s[j] + 32] : 0u;
+    }
+#pragma unroll
+    for (int j = 0; j < kAtOnce; j++) {
+      if ((uint32_t)lane < k[j]) col[o[j]] = (int64_t)v[j];
+      if ((uint32_t)lane + 32u < k[j]) col[o[j] + 32] = (int64_t)v2[j];
+    }
   }
 }
 
-__global__ void __launch_bounds__(kBuildBlock) csr_emit_long_kernel(const int64_t* __restrict__ raw_rowptr,
-                                                                    const uint32_t* __restrict__ raw_col,
-                                                                    const int64_t* __restrict__ rowptr,
-                                                                    const uint32_t* __restrict__ long_rows,
-                                                                    const unsigned long long* __restrict__ long_count,
-                                                                    int64_t* __restrict__ col) {
-  const unsigned long long rows = *long_count;
-  for (unsigned long long w = blockIdx.x; w < rows; w += gridDim.x) {
-    const uint32_t r = long_rows[w];
+// THREADS per listed row: a warp or the block.
+template <int THREADS>
+__global__ void __launch_bounds__(kBuildBlock) csr_emit_listed_kernel(const int64_t* __restrict__ raw_rowptr,
+                                                                      const uint32_t* __restrict__ raw_col,
+                                                                      const int64_t* __restrict__ rowptr,
+                                                                      const uint32_t* __restrict__ listed,
+                                                                      const unsigned long long* __restrict__ count,
+                                                                      int64_t* __restrict__ col) {
+  constexpr int kTeams = kBuildBlock / THREADS;
+  const unsigned long long rows = *count;
+  for (unsigned long long w = (unsigned long long)blockIdx.x * kTeams + threadIdx.x / THREADS; w < rows;
+       w += (unsigned long long)gridDim.x * kTeams) {
+    const uint32_t r = listed[w];
     const int64_t s = raw_rowptr[r], o = rowptr[r];
-    const int64_t k = rowptr[r + 1] - o;
-    for (int64_t j = threadIdx.x; j < k; j += kBuildBlock) col[o + j] = (int64_t)raw_col[s + j];
+    const uint32_t k = (uint32_t)(rowptr[r + 1] - o);
+#pragma unroll 4
+    for (uint32_t j = threadIdx.x % THREADS; j < k; j += THREADS) col[o + j] = (int64_t)raw_col[s + j];
   }
 }
 
 // ---- scratch layout ----------------------------------------------------------------------------------
 struct BuildLayout {
-  size_t counters, raw_rowptr, tile_sums, raw_col, tmp, medium_rows, long_rows, list_counts, total;
+  size_t counters, raw_rowptr, tile_sums, raw_col, tmp, medium_rows, wide_rows, long_rows, list_counts, total;
 };
+
+// Counters of up to 64 MB (2^24 nodes) are spread; beyond, they miss L2 whatever their order, and edge lists sorted by node
+// keep theirs.
+CounterPlace counter_place(int64_t num_nodes) {
+  uint32_t size = 1;
+  while (size < (1u << 24) && (int64_t)size < num_nodes) size <<= 1;
+  return CounterPlace{(int64_t)size < num_nodes ? 0u : size - 1u};
+}
+
+size_t counter_bytes(int64_t num_nodes) {
+  const CounterPlace place = counter_place(num_nodes);
+  return (place.mask ? (size_t)place.mask + 1 : (size_t)num_nodes) * 4;
+}
 
 size_t align_up(size_t x) { return (x + 255) & ~size_t(255); }
 
@@ -442,14 +593,15 @@ BuildLayout build_layout(int64_t m, int64_t num_nodes, uint32_t options) {
   const size_t tiles = ((size_t)num_nodes + kScanTile - 1) / kScanTile + 1;
   BuildLayout L{};
   size_t at = 0;
-  L.counters = at;   at += align_up((size_t)num_nodes * 4 + 4);
+  L.counters = at;   at += align_up(counter_bytes(num_nodes) + 4);
   L.raw_rowptr = at; at += align_up(((size_t)num_nodes + 1) * 8);
   L.tile_sums = at;  at += align_up(tiles * 8);
   L.raw_col = at;    at += align_up(slots * 4 + 4);
   L.tmp = at;        at += align_up(slots * 4 + 4);
   L.medium_rows = at; at += align_up((slots / (kSmallRow + 1) + 1) * 4);
-  L.long_rows = at;   at += align_up((slots / (kMediumRow + 1) + 1) * 4);
-  L.list_counts = at; at += align_up(16);
+  L.wide_rows = at;   at += align_up((slots / (kMediumRow + 1) + 1) * 4);
+  L.long_rows = at;   at += align_up((slots / (kWideRow + 1) + 1) * 4);
+  L.list_counts = at; at += align_up(24);
   L.total = at;
   return L;
 }
@@ -465,18 +617,18 @@ int check_build_args(int64_t m, int64_t num_nodes, uint32_t options) {
   return WALK_B200_OK;
 }
 
-int scan_counts(uint32_t* counts, int64_t n, uint64_t* tile_sums, int64_t* out, bool ends, cudaStream_t s) {
+int scan_counts(uint32_t* counts, int64_t n, CounterPlace place, uint64_t* tile_sums, int64_t* out, bool ends, cudaStream_t s) {
   if (n == 0) {
     WALK_CUDA_TRY(cudaMemsetAsync(out, 0, 8, s));
     return WALK_B200_OK;
   }
   const int64_t tiles = (n + kScanTile - 1) / kScanTile;
-  scan_tile_sums_kernel<<<(unsigned)tiles, kBuildBlock, 0, s>>>(counts, n, tile_sums);
+  scan_tile_sums_kernel<<<(unsigned)tiles, kBuildBlock, 0, s>>>(counts, n, place, tile_sums);
   if (int rc = host::check_launch("scan_tile_sums_kernel")) return rc;
   scan_tile_offsets_kernel<<<1, kBuildBlock, 0, s>>>(tile_sums, tiles);
   if (int rc = host::check_launch("scan_tile_offsets_kernel")) return rc;
-  if (ends) scan_write_kernel<true><<<(unsigned)tiles, kBuildBlock, 0, s>>>(counts, n, tile_sums, out);
-  else scan_write_kernel<false><<<(unsigned)tiles, kBuildBlock, 0, s>>>(counts, n, tile_sums, out);
+  if (ends) scan_write_kernel<true><<<(unsigned)tiles, kBuildBlock, 0, s>>>(counts, n, place, tile_sums, out);
+  else scan_write_kernel<false><<<(unsigned)tiles, kBuildBlock, 0, s>>>(counts, n, place, tile_sums, out);
   return host::check_launch("scan_write_kernel");
 }
 
@@ -522,47 +674,62 @@ int walk_b200_csr_build(const int64_t* src, const int64_t* dst, int64_t num_inpu
   uint32_t* raw_col = reinterpret_cast<uint32_t*>(base + L.raw_col);
   uint32_t* tmp = reinterpret_cast<uint32_t*>(base + L.tmp);
   uint32_t* medium_rows = reinterpret_cast<uint32_t*>(base + L.medium_rows);
+  uint32_t* wide_rows = reinterpret_cast<uint32_t*>(base + L.wide_rows);
   uint32_t* long_rows = reinterpret_cast<uint32_t*>(base + L.long_rows);
   unsigned long long* list_counts = reinterpret_cast<unsigned long long*>(base + L.list_counts);
-  unsigned long long* long_count = list_counts + 1;
+  const unsigned long long *wide_count = list_counts + 1, *long_count = list_counts + 2;
 
   if (num_nodes == 0 || num_input_edges == 0) {
     WALK_CUDA_TRY(cudaMemsetAsync(rowptr, 0, ((size_t)num_nodes + 1) * 8, s));
     return WALK_B200_OK;
   }
-  WALK_CUDA_TRY(cudaMemsetAsync(counters, 0, (size_t)num_nodes * 4, s));
-  WALK_CUDA_TRY(cudaMemsetAsync(list_counts, 0, 16, s));
+  const CounterPlace place = counter_place(num_nodes);
+  WALK_CUDA_TRY(cudaMemsetAsync(counters, 0, counter_bytes(num_nodes), s));
+  WALK_CUDA_TRY(cudaMemsetAsync(list_counts, 0, 24, s));
 
   const unsigned edge_grid = capped_grid((num_input_edges + kBuildBlock - 1) / kBuildBlock, 16);
-  csr_edges_kernel<false><<<edge_grid, kBuildBlock, 0, s>>>(src, dst, num_input_edges, num_nodes, options, counters,
+  csr_edges_kernel<false><<<edge_grid, kBuildBlock, 0, s>>>(src, dst, num_input_edges, num_nodes, options, place, counters,
                                                             nullptr, status_flags);
   if (int rc = host::check_launch("csr_edges_kernel<count>")) return rc;
-  if (int rc = scan_counts(counters, num_nodes, tile_sums, raw_rowptr, true, s)) return rc;
-  csr_edges_kernel<true><<<edge_grid, kBuildBlock, 0, s>>>(src, dst, num_input_edges, num_nodes, options, counters,
+  if (int rc = scan_counts(counters, num_nodes, place, tile_sums, raw_rowptr, true, s)) return rc;
+  csr_edges_kernel<true><<<edge_grid, kBuildBlock, 0, s>>>(src, dst, num_input_edges, num_nodes, options, place, counters,
                                                            raw_col, status_flags);
   if (int rc = host::check_launch("csr_edges_kernel<fill>")) return rc;
 
-  const unsigned row_grid = capped_grid((num_nodes + kBuildWarps - 1) / kBuildWarps, 16);
+  const unsigned row_grid = (unsigned)((num_nodes + kBuildBlock - 1) / kBuildBlock);  // a warp per 32 rows
   csr_sort_small_kernel<<<row_grid, kBuildBlock, 0, s>>>(raw_rowptr, num_nodes, options, raw_col, counters, medium_rows,
-                                                         long_rows, list_counts);
+                                                         wide_rows, long_rows, list_counts);
   if (int rc = host::check_launch("csr_sort_small_kernel")) return rc;
-  int key_bits = 1;
-  while (key_bits < 31 && (1ll << key_bits) < num_nodes) key_bits++;
-  const int passes = (key_bits + 7) / 8;
-  const int digit_bits = (key_bits + passes - 1) / passes;
-  const unsigned long_grid = (unsigned)host::sm_count() * 8;
-  csr_sort_medium_kernel<<<long_grid, kBuildBlock, 0, s>>>(raw_rowptr, options, passes, digit_bits, raw_col, tmp, counters,
-                                                           medium_rows, list_counts);
-  if (int rc = host::check_launch("csr_sort_medium_kernel")) return rc;
-  csr_sort_long_kernel<<<long_grid, kBuildBlock, 0, s>>>(raw_rowptr, options, passes, digit_bits, raw_col, tmp, counters,
-                                                         long_rows, long_count);
-  if (int rc = host::check_launch("csr_sort_long_kernel")) return rc;
+  const unsigned list_grid = (unsigned)host::sm_count() * 8;
+  csr_sort_listed_kernel<false><<<list_grid, kBuildBlock, 0, s>>>(raw_rowptr, options, raw_col, counters, medium_rows, list_counts);
+  if (int rc = host::check_launch("csr_sort_listed_kernel<false>")) return rc;
+  csr_sort_listed_kernel<true><<<list_grid, kBuildBlock, 0, s>>>(raw_rowptr, options, raw_col, counters, wide_rows, wide_count);
+  if (int rc = host::check_launch("csr_sort_listed_kernel<true>")) return rc;
+  if ((options & WALK_B200_BUILD_DEDUPE) && num_nodes <= (1ll << kBitmapBits)) {
+    constexpr int kBitmapBytes = 1 << (kBitmapBits - 3);
+    WALK_CUDA_TRY(cudaFuncSetAttribute(csr_bitmap_long_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kBitmapBytes));
+    csr_bitmap_long_kernel<<<(unsigned)host::sm_count(), kBitmapBlock, kBitmapBytes, s>>>(raw_rowptr, raw_col, counters,
+                                                                                         long_rows, long_count);
+    if (int rc = host::check_launch("csr_bitmap_long_kernel")) return rc;
+  } else {
+    int key_bits = 1;
+    while (key_bits < 31 && (1ll << key_bits) < num_nodes) key_bits++;
+    const int passes = (key_bits + 7) / 8;
+    const int digit_bits = (key_bits + passes - 1) / passes;
+    csr_sort_long_kernel<<<list_grid, kBuildBlock, 0, s>>>(raw_rowptr, options, passes, digit_bits, raw_col, tmp, counters,
+                                                           long_rows, long_count);
+    if (int rc = host::check_launch("csr_sort_long_kernel")) return rc;
+  }
 
-  if (int rc = scan_counts(counters, num_nodes, tile_sums, rowptr, false, s)) return rc;
+  if (int rc = scan_counts(counters, num_nodes, CounterPlace{0}, tile_sums, rowptr, false, s)) return rc;
   csr_emit_small_kernel<<<row_grid, kBuildBlock, 0, s>>>(raw_rowptr, raw_col, rowptr, num_nodes, col);
   if (int rc = host::check_launch("csr_emit_small_kernel")) return rc;
-  csr_emit_long_kernel<<<long_grid, kBuildBlock, 0, s>>>(raw_rowptr, raw_col, rowptr, long_rows, long_count, col);
-  return host::check_launch("csr_emit_long_kernel");
+  csr_emit_listed_kernel<32><<<list_grid, kBuildBlock, 0, s>>>(raw_rowptr, raw_col, rowptr, medium_rows, list_counts, col);
+  if (int rc = host::check_launch("csr_emit_listed_kernel<32>")) return rc;
+  csr_emit_listed_kernel<kBuildBlock><<<list_grid, kBuildBlock, 0, s>>>(raw_rowptr, raw_col, rowptr, wide_rows, wide_count, col);
+  if (int rc = host::check_launch("csr_emit_listed_kernel<256>")) return rc;
+  csr_emit_listed_kernel<kBuildBlock><<<list_grid, kBuildBlock, 0, s>>>(raw_rowptr, raw_col, rowptr, long_rows, long_count, col);
+  return host::check_launch("csr_emit_listed_kernel<256>");
 }
 
 }  // extern "C"

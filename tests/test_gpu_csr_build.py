@@ -93,3 +93,37 @@ def test_degenerate_inputs(cuda):
     rp, cl = build([0, 1, 9], [1, 2, 0], 4, check=False)  # the bad edge is left out
     np.testing.assert_array_equal(rp, [0, 1, 3, 4, 4])
     np.testing.assert_array_equal(cl, [1, 0, 2, 1])
+
+
+@pytest.mark.parametrize("symmetrize", [True, False])
+@pytest.mark.parametrize("n", [1, 2, 3, 31, 32, 33, 4096, 4097, 1 << 24, (1 << 24) + 1])
+def test_node_counts_around_the_counter_spread(cuda, n, symmetrize):
+    """Counters are spread over a power of two, and left in node order beyond 2^24 nodes; rows come 32 to a warp."""
+    rng = np.random.default_rng(n)
+    m = 5000
+    src, dst = (rng.random(m) ** 4 * n).astype(np.int64), rng.integers(0, n, m)
+    kw = dict(symmetrize=symmetrize, drop_self_loops=False, dedupe=True)
+    rp, cl = build(src, dst, n, **kw)
+    want_rp, want_cl = numpy_csr(src, dst, n, **kw)
+    np.testing.assert_array_equal(rp, want_rp)
+    np.testing.assert_array_equal(cl, want_cl)
+
+
+@pytest.mark.parametrize("n", [5000, 1 << 20, (1 << 20) + 33, (1 << 22) + 5])
+def test_sorted_by_registers_bitmap_or_radix(cuda, n):
+    """Row lengths around each kernel's limits; with few columns, exactly a bitmap of them, a word more
+    and far more (radix sort). Dense, sparse and one-column rows."""
+    rng = np.random.default_rng(n)
+    lengths = [129, 256, 257, 511, 512, 513, 1023, 1024, 1025, 2047, 2048, 2049, 2050, 4096, 5000, 60000]
+    src, dst = [], []
+    for r, d in enumerate(lengths):
+        for k, span in enumerate((n, min(n, d + 3), 1)):
+            src.append(np.full(d, (7 * r + k) % n, np.int64))
+            dst.append(n - 1 - rng.integers(0, span, d))
+    src, dst = np.concatenate(src), np.concatenate(dst)
+    perm = rng.permutation(src.size)
+    for dedupe in (True, False):
+        rp, cl = build(src[perm], dst[perm], n, symmetrize=False, drop_self_loops=False, dedupe=dedupe)
+        want_rp, want_cl = numpy_csr(src, dst, n, False, False, dedupe)
+        np.testing.assert_array_equal(rp, want_rp)
+        np.testing.assert_array_equal(cl, want_cl)
