@@ -186,6 +186,11 @@ int walk_b200_rowdesc_pack(const int64_t* rowptr, int64_t num_nodes, int64_t num
 int walk_b200_edgeset_buckets(int64_t num_edges, uint64_t* buckets);
 int walk_b200_edgeset_build(const walk_b200_csr* g, uint64_t* table, uint64_t buckets,
                             uint32_t* status_flags, void* stream);
+/* The same set, built faster with scratch (a little over 8 bytes per edge, 128-byte aligned; free when the build is done):
+ * tables larger than L2 are filled piece by piece. *bytes = 0 where scratch would not help; scratch NULL is allowed. */
+int walk_b200_edgeset_scratch_bytes(int64_t num_edges, uint64_t buckets, uint64_t* bytes);
+int walk_b200_edgeset_build_binned(const walk_b200_csr* g, uint64_t* table, uint64_t buckets, void* scratch,
+                                   uint64_t scratch_bytes, uint32_t* status_flags, void* stream);
 
 /*
  * Fused edge records for the uniform walk: fused[e] = (col[e], row descriptor of col[e]), 16 bytes per

@@ -667,6 +667,65 @@ int grid_for_edge_chunks(int64_t n) {
   return (int)(b < cap ? b : cap);
 }
 
+// How the edge hash set's build sorts its keys (edgeset_bin_kernel): pieces of the table of at most 32 MB, so that the one
+// being filled and the next stay in L2 beside the streams; not at all while the whole table is at most 64 MB.
+struct EdgeBins {
+  int bits = 0;        // 0: no bins
+  uint64_t room = 0;   // keys per bin
+  uint64_t bytes = 0;  // scratch: the bins' cursors, then their keys
+};
+
+EdgeBins edge_bins(int64_t num_edges, uint64_t buckets) {
+  EdgeBins b;
+  const uint64_t table = buckets > (UINT64_MAX >> 5) ? UINT64_MAX : buckets * 32;
+  if (num_edges == 0 || table <= (64ull << 20)) return b;
+  while ((1 << b.bits) < kEdgeMaxBins && (table >> b.bits) > (32ull << 20)) b.bits++;
+  const double even = std::ceil((double)num_edges / (double)(1 << b.bits));
+  b.room = ((uint64_t)(even + 8.0 * std::sqrt(even)) + 256) / 256 * 256;  // eight standard deviations
+  b.bytes = (uint64_t)(1 << b.bits) * (kEdgeCursorPitch * 8 + b.room * 8);
+  return b;
+}
+
+int edgeset_build_impl(const walk_b200_csr* g, uint64_t* table, uint64_t buckets, void* scratch, uint64_t scratch_bytes,
+                       uint32_t* status_flags, void* stream) {
+  if (int rc = check_csr(g)) return rc;
+  if (!table || buckets == 0) return fail(WALK_B200_ERR_INVALID_ARG, "edge set table is NULL or empty");
+  if ((reinterpret_cast<uintptr_t>(table) & 31) != 0)
+    return fail(WALK_B200_ERR_INVALID_ARG, "edge set table must be 32-byte aligned");
+  if (g->num_nodes >= 0xffffffffll)
+    return fail(WALK_B200_ERR_UNSUPPORTED, "the edge hash set needs num_nodes < 2^32 - 1");
+  if (buckets * kEdgeSlotsPerBucket < (uint64_t)g->num_edges + (uint64_t)g->num_edges / 4)
+    return fail(WALK_B200_ERR_INVALID_ARG, "edge set table too small: %llu buckets for %lld edges",
+                (unsigned long long)buckets, (long long)g->num_edges);
+  EdgeBins bins;
+  if (scratch) {
+    bins = edge_bins(g->num_edges, buckets);
+    if (scratch_bytes < bins.bytes || (reinterpret_cast<uintptr_t>(scratch) & 127) != 0)
+      return fail(WALK_B200_ERR_INVALID_ARG, "edge set scratch: %llu bytes given, %llu needed, 128-byte aligned",
+                  (unsigned long long)scratch_bytes, (unsigned long long)bins.bytes);
+  }
+  cudaStream_t s = (cudaStream_t)stream;
+  unsigned long long* slots = reinterpret_cast<unsigned long long*>(table);
+  CUDA_TRY(cudaMemsetAsync(table, 0xff, buckets * kEdgeSlotsPerBucket * sizeof(uint64_t), s));
+  if (g->num_edges == 0) return WALK_B200_OK;
+  if (bins.bits == 0) {
+    edgeset_build_kernel<<<grid_for_edge_chunks(g->num_edges), kBlock, 0, s>>>(g->rowptr, g->col, g->num_nodes, g->num_edges,
+                                                                               slots, buckets, status_flags);
+    return check_launch("edgeset_build_kernel");
+  }
+  const size_t cursor_bytes = (size_t)kEdgeCursorPitch * 8 << bins.bits;
+  unsigned long long* cursors = static_cast<unsigned long long*>(scratch);
+  uint64_t* binned = reinterpret_cast<uint64_t*>(static_cast<char*>(scratch) + cursor_bytes);
+  CUDA_TRY(cudaMemsetAsync(cursors, 0, cursor_bytes, s));
+  edgeset_bin_kernel<<<grid_for_edge_chunks(g->num_edges), kBlock, 0, s>>>(
+      g->rowptr, g->col, g->num_nodes, g->num_edges, bins.bits, bins.room, cursors, binned, slots, buckets, status_flags);
+  if (int rc = check_launch("edgeset_bin_kernel")) return rc;
+  const uint64_t tiles = (bins.room + kEdgeTile - 1) / kEdgeTile;
+  edgeset_insert_kernel<<<(unsigned)(tiles << bins.bits), kBlock, 0, s>>>(binned, bins.room, (uint32_t)tiles, cursors, slots,
+                                                                          buckets, status_flags);
+  return check_launch("edgeset_insert_kernel");
+}
+
 // Rows of a matrix per block of the tile kernels: what the tile holds, but no fewer blocks than fill the device.
 uint32_t tile_rows(int64_t num_rows, int64_t row_len) {
   int64_t r = kTileEntries / row_len;
@@ -876,20 +935,18 @@ int walk_b200_edgeset_buckets(int64_t num_edges, uint64_t* buckets) {
 
 int walk_b200_edgeset_build(const walk_b200_csr* g, uint64_t* table, uint64_t buckets,
                             uint32_t* status_flags, void* stream) {
-  if (int rc = check_csr(g)) return rc;
-  if (!table || buckets == 0) return fail(WALK_B200_ERR_INVALID_ARG, "edge set table is NULL or empty");
-  if ((reinterpret_cast<uintptr_t>(table) & 31) != 0)
-    return fail(WALK_B200_ERR_INVALID_ARG, "edge set table must be 32-byte aligned");
-  if (g->num_nodes >= 0xffffffffll)
-    return fail(WALK_B200_ERR_UNSUPPORTED, "the edge hash set needs num_nodes < 2^32 - 1");
-  if (buckets * kEdgeSlotsPerBucket < (uint64_t)g->num_edges + (uint64_t)g->num_edges / 4)
-    return fail(WALK_B200_ERR_INVALID_ARG, "edge set table too small: %llu buckets for %lld edges",
-                (unsigned long long)buckets, (long long)g->num_edges);
-  CUDA_TRY(cudaMemsetAsync(table, 0xff, buckets * kEdgeSlotsPerBucket * sizeof(uint64_t), (cudaStream_t)stream));
-  if (g->num_edges == 0) return WALK_B200_OK;
-  edgeset_build_kernel<<<grid_for_streaming(g->num_edges), kBlock, 0, (cudaStream_t)stream>>>(
-      g->rowptr, g->col, g->num_nodes, g->num_edges, (unsigned long long*)table, buckets, status_flags);
-  return check_launch("edgeset_build_kernel");
+  return edgeset_build_impl(g, table, buckets, nullptr, 0, status_flags, stream);
+}
+
+int walk_b200_edgeset_scratch_bytes(int64_t num_edges, uint64_t buckets, uint64_t* bytes) {
+  if (num_edges < 0 || !bytes) return fail(WALK_B200_ERR_INVALID_ARG, "bad edge count or NULL result");
+  *bytes = edge_bins(num_edges, buckets).bytes;
+  return WALK_B200_OK;
+}
+
+int walk_b200_edgeset_build_binned(const walk_b200_csr* g, uint64_t* table, uint64_t buckets, void* scratch,
+                                   uint64_t scratch_bytes, uint32_t* status_flags, void* stream) {
+  return edgeset_build_impl(g, table, buckets, scratch, scratch_bytes, status_flags, stream);
 }
 
 int walk_b200_fused_build(const walk_b200_csr* g, void* fused, uint32_t* status_flags, void* stream) {

@@ -582,12 +582,14 @@ constexpr int kEdgeMaxProbe = 4096;  // buckets; far beyond anything a half-full
 
 __host__ __device__ __forceinline__ uint64_t edge_key(uint64_t x, uint64_t t) { return (x << 32) | t; }
 
+__device__ __forceinline__ uint64_t edge_hash(uint64_t key) {
+  key ^= key >> 30; key *= 0xbf58476d1ce4e5b9ull;
+  key ^= key >> 27; key *= 0x94d049bb133111ebull;
+  return key ^ (key >> 31);
+}
+
 __device__ __forceinline__ uint64_t edge_bucket(uint64_t key, uint64_t num_buckets) {
-  uint64_t z = key;
-  z ^= z >> 30; z *= 0xbf58476d1ce4e5b9ull;
-  z ^= z >> 27; z *= 0x94d049bb133111ebull;
-  z ^= z >> 31;
-  return __umul64hi(z, num_buckets);
+  return __umul64hi(edge_hash(key), num_buckets);
 }
 
 // ---- source rows of consecutive edges ------------------------------------------------------
@@ -617,35 +619,115 @@ __device__ __forceinline__ int64_t row_of(const int64_t* __restrict__ rowptr, in
 // lies in, and a lane then looks its own row up among those few (their bounds stay in L1) instead of among all rows.
 constexpr int kEdgeChunk = 256;
 
+__device__ __forceinline__ void edge_insert(unsigned long long* __restrict__ table, uint64_t num_buckets, uint64_t key, uint32_t* flags) {
+  uint64_t b = edge_bucket(key, num_buckets);
+  for (int probe = 0; probe < kEdgeMaxProbe; probe++) {
+    unsigned long long* slot = table + b * kEdgeSlotsPerBucket;
+#pragma unroll
+    for (int k = 0; k < kEdgeSlotsPerBucket; k++) {
+      const unsigned long long old = atomicCAS(slot + k, kEdgeEmpty, key);
+      if (old == kEdgeEmpty || old == key) return;
+    }
+    if (++b == num_buckets) b = 0;
+  }
+  raise_flag(flags, WALK_B200_FLAG_EDGESET_FULL);
+}
+
+// Tables that stay in L2: every edge goes straight to its bucket.
 __global__ void __launch_bounds__(kBlock) edgeset_build_kernel(const int64_t* __restrict__ rowptr,
                                                                const int64_t* __restrict__ col,
                                                                int64_t num_nodes, int64_t num_edges,
                                                                unsigned long long* __restrict__ table,
                                                                uint64_t num_buckets, uint32_t* flags) {
-  const int64_t stride = (int64_t)gridDim.x * kBlock;
-  for (int64_t e = (int64_t)blockIdx.x * kBlock + threadIdx.x; e < num_edges; e += stride) {
-    // source row of edge e: last v with rowptr[v] <= e
-    int64_t lo = 0, hi = num_nodes;
-    while (hi - lo > 1) {
-      const int64_t mid = lo + (hi - lo) / 2;
-      if (__ldg(rowptr + mid) <= e) lo = mid; else hi = mid;
+  const int64_t warps = (int64_t)gridDim.x * kWarpsPerBlock;
+  for (int64_t c = (int64_t)blockIdx.x * kWarpsPerBlock + (threadIdx.x >> 5); c * kEdgeChunk < num_edges; c += warps) {
+    const int64_t first = c * kEdgeChunk, end = min(first + kEdgeChunk, num_edges);
+    const int64_t row_lo = warp_row_of(rowptr, 0, num_nodes, first);
+    const int64_t row_hi = warp_row_of(rowptr, row_lo, num_nodes, end - 1) + 1;
+    for (int64_t e = first + (threadIdx.x & 31); e < end; e += 32) {
+      const int64_t t = __ldg(col + e);
+      if ((uint64_t)t >= (uint64_t)num_nodes) { raise_flag(flags, WALK_B200_FLAG_BAD_NODE); continue; }
+      edge_insert(table, num_buckets, edge_key((uint64_t)row_of(rowptr, row_lo, row_hi, e), (uint64_t)t), flags);
     }
-    const int64_t t = __ldg(col + e);
-    if ((uint64_t)t >= (uint64_t)num_nodes) { raise_flag(flags, WALK_B200_FLAG_BAD_NODE); continue; }
-    const uint64_t key = edge_key((uint64_t)lo, (uint64_t)t);
-    uint64_t b = edge_bucket(key, num_buckets);
-    bool placed = false;
-    for (int probe = 0; probe < kEdgeMaxProbe && !placed; probe++) {
-      unsigned long long* slot = table + b * kEdgeSlotsPerBucket;
-#pragma unroll
-      for (int k = 0; k < kEdgeSlotsPerBucket && !placed; k++) {
-        const unsigned long long old = atomicCAS(slot + k, kEdgeEmpty, key);
-        if (old == kEdgeEmpty || old == key) placed = true;
-      }
-      if (++b == num_buckets) b = 0;
-    }
-    if (!placed) raise_flag(flags, WALK_B200_FLAG_EDGESET_FULL);
   }
+}
+
+// Larger tables: an insert is a random read-modify-write of DRAM there, and its rate bounds the build (R-MAT 20, a table of
+// 1 GB: 1500 us). So the keys are first sorted into 2^bin_bits bins by the top bits of their hash, which order the buckets
+// too: a bin's keys fall into one piece of the table, small enough to stay in L2 while the bin is inserted. Two streaming
+// passes over 8 bytes per edge and one over the table: 388 + 771 us. A bin is given room for what a hash spreads into it; keys
+// beyond that (many copies of one edge) go straight to the table.
+constexpr int kEdgeMaxBins = 512;
+constexpr int kEdgeCursorPitch = 16;  // 8-byte words between two bins' cursors: a line each
+constexpr int kEdgeTile = kEdgeChunk * kWarpsPerBlock;
+
+__global__ void __launch_bounds__(kBlock) edgeset_bin_kernel(const int64_t* __restrict__ rowptr, const int64_t* __restrict__ col,
+                                                             int64_t num_nodes, int64_t num_edges, int bin_bits, uint64_t room,
+                                                             unsigned long long* __restrict__ cursors,
+                                                             uint64_t* __restrict__ binned,
+                                                             unsigned long long* __restrict__ table, uint64_t num_buckets,
+                                                             uint32_t* flags) {
+  constexpr int kPer = kEdgeChunk / 32;
+  __shared__ uint32_t held[kEdgeMaxBins];
+  __shared__ unsigned long long base[kEdgeMaxBins];
+  const int lane = threadIdx.x & 31, bins = 1 << bin_bits;
+  for (int64_t tile = blockIdx.x; tile * kEdgeTile < num_edges; tile += gridDim.x) {
+    for (int b = threadIdx.x; b < bins; b += kBlock) held[b] = 0;
+    __syncthreads();
+    uint64_t key[kPer];
+    uint32_t rank[kPer];
+    const int64_t first = tile * kEdgeTile + (threadIdx.x >> 5) * kEdgeChunk, end = min(first + kEdgeChunk, num_edges);
+    if (first < num_edges) {
+      const int64_t row_lo = warp_row_of(rowptr, 0, num_nodes, first);
+      const int64_t row_hi = warp_row_of(rowptr, row_lo, num_nodes, end - 1) + 1;
+#pragma unroll
+      for (int k = 0; k < kPer; k++) {
+        const int64_t e = first + 32 * k + lane;
+        key[k] = kEdgeEmpty;
+        if (e >= end) continue;
+        const int64_t t = __ldg(col + e);
+        if ((uint64_t)t >= (uint64_t)num_nodes) { raise_flag(flags, WALK_B200_FLAG_BAD_NODE); continue; }
+        key[k] = edge_key((uint64_t)row_of(rowptr, row_lo, row_hi, e), (uint64_t)t);
+        rank[k] = atomicAdd(&held[edge_hash(key[k]) >> (64 - bin_bits)], 1u);
+      }
+    } else {
+#pragma unroll
+      for (int k = 0; k < kPer; k++) key[k] = kEdgeEmpty;
+    }
+    __syncthreads();
+    for (int b = threadIdx.x; b < bins; b += kBlock)
+      if (held[b]) base[b] = atomicAdd(cursors + b * kEdgeCursorPitch, (unsigned long long)held[b]);
+    __syncthreads();
+#pragma unroll
+    for (int k = 0; k < kPer; k++) {
+      if (key[k] == kEdgeEmpty) continue;
+      const uint32_t b = (uint32_t)(edge_hash(key[k]) >> (64 - bin_bits));
+      const uint64_t at = base[b] + rank[k];
+      if (at < room) binned[(uint64_t)b * room + at] = key[k];
+      else edge_insert(table, num_buckets, key[k], flags);
+    }
+  }
+}
+
+// Blocks start in order, so those in flight work on one bin or two.
+__global__ void __launch_bounds__(kBlock) edgeset_insert_kernel(const uint64_t* __restrict__ binned, uint64_t room,
+                                                                uint32_t tiles_per_bin,
+                                                                const unsigned long long* __restrict__ cursors,
+                                                                unsigned long long* __restrict__ table, uint64_t num_buckets,
+                                                                uint32_t* flags) {
+  constexpr int kPer = kEdgeTile / kBlock;
+  const uint32_t bin = blockIdx.x / tiles_per_bin;
+  const uint64_t from = (uint64_t)(blockIdx.x - bin * tiles_per_bin) * kEdgeTile + threadIdx.x;
+  const uint64_t filled = min((uint64_t)cursors[(size_t)bin * kEdgeCursorPitch], room);
+  uint64_t key[kPer];
+#pragma unroll
+  for (int k = 0; k < kPer; k++) {
+    const uint64_t i = from + (uint64_t)k * kBlock;
+    key[k] = i < filled ? __ldcs(reinterpret_cast<const unsigned long long*>(binned) + (uint64_t)bin * room + i) : kEdgeEmpty;
+  }
+#pragma unroll
+  for (int k = 0; k < kPer; k++)
+    if (key[k] != kEdgeEmpty) edge_insert(table, num_buckets, key[k], flags);
 }
 
 // ---------------------------------------------------------------------------------

@@ -246,10 +246,19 @@ class WalkGraph:
                 if want * 32 + 12 * self.num_edges < (free + cached) // 2:
                     buckets = want
             table = torch.empty(buckets * 4, dtype=torch.int64, device=self.device)
+            # scratch of about 8 bytes per edge speeds the build up; what the reverse positions take next (12) covers it
+            need = _lib.edgeset_scratch_bytes(self.num_edges, buckets)
+            if need:
+                free, _ = torch.cuda.mem_get_info(self.device)
+                cached = torch.cuda.memory_reserved(self.device) - torch.cuda.memory_allocated(self.device)
+                need = need if need + (256 << 20) < free + cached else 0
+            scratch = torch.empty(need, dtype=torch.uint8, device=self.device) if need else None
             csr = self.csr()
-            _lib.check(_lib.lib().walk_b200_edgeset_build(C.byref(csr), table.data_ptr(), buckets,
-                                                          self.flags.data_ptr(), _stream_handle(stream, self.device)))
+            _lib.check(_lib.lib().walk_b200_edgeset_build_binned(C.byref(csr), table.data_ptr(), buckets,
+                                                                 scratch.data_ptr() if need else None, need,
+                                                                 self.flags.data_ptr(), _stream_handle(stream, self.device)))
             f = _take_flags(self.flags, stream, self.device)
+            del scratch
             if f:
                 raise ValueError(f"edge set build failed, status flags 0x{f:x}: {describe_flags(f)}")
             self.edgeset_buckets = buckets

@@ -53,3 +53,40 @@ def test_unsorted_rows_are_seen(cuda):
     graph = WalkGraph(torch.tensor([0, 3, 3, 3]).to(cuda), torch.from_numpy(ok).to(cuda), edgeset=True)
     assert graph.rows_sorted is True and graph.colrev is not None
     assert _lib.last_kernel() == "colrev_build_kernel"
+
+
+@pytest.mark.parametrize("edges,copies,buckets", [(1, 1, (2 << 20) + 1), (2049, 1, 4 << 20), (300000, 1, 5000011), (300000, 3, 4 << 20),
+                                                  (7, 50000, 4 << 20), (300000, 1, (1 << 28) + 1)])
+def test_edge_set_built_by_bins_holds_the_same_members(cuda, edges, copies, buckets):
+    """Tables beyond L2 are filled bin by bin (4 to 512 bins here); copies of an edge overflow their bin and go in directly."""
+    rng = np.random.default_rng(edges)
+    nodes = 4000
+    rowptr, pairs = _csr(nodes, (rng.random((edges, 2)) ** 2 * nodes).astype(np.int64))
+    col = torch.from_numpy(np.repeat(pairs[:, 1], copies)).to(cuda)
+    rp = torch.from_numpy(rowptr * copies).to(cuda)
+    csr = _lib.Csr(rp.data_ptr(), col.data_ptr(), nodes, col.numel(), None, 0, 0, None, 0)
+    need = _lib.edgeset_scratch_bytes(col.numel(), buckets)
+    assert need >= 8 * col.numel()
+    table = torch.empty(buckets * 4, dtype=torch.int64, device=cuda)
+    scratch = torch.empty(need, dtype=torch.uint8, device=cuda)
+    flags = torch.zeros(1, dtype=torch.int32, device=cuda)
+    stream = torch.cuda.current_stream(cuda).cuda_stream
+    _lib.check(_lib.lib().walk_b200_edgeset_build_binned(csr, table.data_ptr(), buckets, scratch.data_ptr(), need, flags.data_ptr(), stream))
+    assert _lib.last_kernel() == "edgeset_insert_kernel" and int(flags) == 0
+    want = torch.from_numpy(pairs[:, 0] << 32 | pairs[:, 1]).to(cuda)
+    used = table != -1
+    assert torch.equal(table[used].sort().values, want.sort().values)
+    # every member within its probe sequence: the buckets between its own and the one it stands in are full
+    z = pairs[:, 0].astype(np.uint64) << np.uint64(32) | pairs[:, 1].astype(np.uint64)
+    z = (z ^ (z >> np.uint64(30))) * np.uint64(0xbf58476d1ce4e5b9)
+    z = (z ^ (z >> np.uint64(27))) * np.uint64(0x94d049bb133111eb)
+    z ^= z >> np.uint64(31)
+    home = {int(k): (int(h) * buckets) >> 64 for k, h in zip(pairs[:, 0] << 32 | pairs[:, 1], z)}
+    at = used.nonzero().flatten()
+    stands = {int(k): int(i) // 4 for k, i in zip(table[at].tolist(), at.tolist())}
+    full = used.view(-1, 4).all(dim=1)
+    for k, h in home.items():
+        if stands[k] != h:
+            assert bool(full[h:stands[k]].all() if stands[k] > h else full[h:].all() & full[:stands[k]].all())
+    assert _lib.lib().walk_b200_edgeset_build_binned(csr, table.data_ptr(), buckets, scratch.data_ptr(), need - 1, None,
+                                                     stream) == _lib.ERR_INVALID_ARG
