@@ -100,14 +100,9 @@ class WalkGraph:
         self.num_nodes = rowptr.numel() - 1
         self.num_edges = col.numel()
         self.symmetric = bool(symmetric)
-        self.rowdesc = None
-        self.edgeset = None
-        self.edgeset_buckets = 0
-        self.colrev = None
-        self.colrev16 = None
-        self.fused = None
-        self.steps = None         # step array (see build_steps) and the field widths of its records (0: uint32 columns)
-        self.steps_bits = 0
+        # the structures, none built yet (steps: see build_steps; steps_bits: the field widths of its records, 0: uint32 columns)
+        self.__dict__.update(rowdesc=None, edgeset=None, edgeset_buckets=0, colrev=None, colrev16=None, fused=None, steps=None,
+                             steps_bits=0)
         self.walk_calls = 0       # walks served: the step array is built on the second
         # size of the edge hash set in 8-byte slots per edge: 2 = half full (the minimum), 4 = a quarter full;
         # None = the library's tuning (default 4), taken when the table fits half of the free device memory
