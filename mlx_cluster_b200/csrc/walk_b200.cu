@@ -557,6 +557,11 @@ int launch_n2v(const Node2vecParams& P, bool sym, cudaStream_t s) {
     if (e) return launch_n2v_kernel(node2vec_walk_kernel<uint32_t, MEMBER_HASH, true, true, false, true>, P, s);
     return launch_n2v_kernel(node2vec_walk_kernel<uint32_t, MEMBER_HASH, true, false, false, true>, P, s);
   }
+  // light rejection (rev_pays says no) on a graph with 4-byte columns; packed records are 8 bytes like col and gain nothing here
+  if (fits32 && member == MEMBER_HASH && P.desc && P.steps && !P.step_bits.id && !P.counters && !kernel_forced()) {
+    if (P.e_out) return launch_n2v_kernel(node2vec_walk_kernel<uint32_t, MEMBER_HASH, true, true, false, false, HOST_NONE, true>, P, s);
+    return launch_n2v_kernel(node2vec_walk_kernel<uint32_t, MEMBER_HASH, true, false, false, false, HOST_NONE, true>, P, s);
+  }
   if (fits32 && g_tuning.n2v_idx.load() != 1) return launch_n2v_i<uint32_t>(P, member, s);
   return launch_n2v_i<int64_t>(P, member, s);
 }

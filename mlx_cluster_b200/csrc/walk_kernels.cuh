@@ -955,10 +955,13 @@ enum : int { HOST_NONE = 0, HOST_NARROW = 1, HOST_WIDE = 2 };
 // rejected without touching memory at all. At (p, q) = (0.25, 4) that is three attempts in four.
 // Same draws, same decisions, fewer gathers.
 //
+// COL32 (hash membership without REV): candidates come from the graph's 4-byte columns, half the array that the gathers
+// miss in. R-MAT 22, every node, 40 steps, (1, 2): 7.32 -> 7.06 ms; left to stay in L2 like other lines, no gain (7.06 of 7.07).
+//
 // HOST (the host-buffer entry point's single-launch mode): finished walks are counted per slab of
 // 2^slab_shift rows, so the host can copy a slab out as soon as its last walk is done; with HOST_NARROW
 // the walk and edge matrices are int32 (P.n_out / P.e_out point at int32 storage; the ids fit).
-template <typename idx_t, int MEMBER, bool USE_DESC, bool HAS_EOUT, bool COUNT, bool REV = false, int HOST = HOST_NONE>
+template <typename idx_t, int MEMBER, bool USE_DESC, bool HAS_EOUT, bool COUNT, bool REV = false, int HOST = HOST_NONE, bool COL32 = false>
 __global__ void __launch_bounds__(kBlock, COUNT ? 1 : 6) node2vec_walk_kernel(const Node2vecParams P) {
   static_assert(!REV || (MEMBER == MEMBER_HASH && USE_DESC && sizeof(idx_t) == 4), "REV needs hash membership, row descriptors, 32-bit indices");
   constexpr unsigned kFull = 0xffffffffu;
@@ -967,6 +970,7 @@ __global__ void __launch_bounds__(kBlock, COUNT ? 1 : 6) node2vec_walk_kernel(co
   const int32_t L = P.walk_length;
   const int64_t n = P.num_walks;
   const int64_t* __restrict__ col = P.col;
+  const uint32_t* __restrict__ col32 = static_cast<const uint32_t*>(P.steps);
 
   // warp-uniform queue of walks: [q_next, q_end) of the current chunk of 32
   const int64_t n_chunks = (n + 31) / 32;
@@ -1152,7 +1156,8 @@ __global__ void __launch_bounds__(kBlock, COUNT ? 1 : 6) node2vec_walk_kernel(co
         h1 = ld16((const char*)addr + 16, policy);
         if (COUNT) c_loads += 4;
       } else {
-        val = ld8(addr, policy);
+        if (COL32 && state == ST_ATTEMPT) val = (int64_t)ld4(col32 + (int64_t)e, policy);
+        else val = ld8(addr, policy);
         const bool pair = !USE_DESC && (state == ST_ROW || state == ST_XROW);
         if (pair) val2 = ld8((const char*)addr + 8, policy);
         // the instrumented kernel's extra look at deg(x) is bookkeeping, not part of the walk

@@ -419,3 +419,28 @@ def test_triangle_filter_at_scale(cuda):
         want = oracle.node2vec_walk(rowptr.cpu().numpy(), col.cpu().numpy(), picked.cpu().numpy(), L, *pq, seed=3,
                                     walk_index_stride=997)
         np.testing.assert_array_equal(got[picked].cpu().numpy(), want)
+
+
+@pytest.mark.parametrize("symmetric", [False, True])
+@pytest.mark.parametrize("p,q", [(1.0, 2.0), (0.5, 1.5), (4.0, 1.25)])
+def test_per_lane_kernel_on_four_byte_columns(cuda, monkeypatch, symmetric, p, q):
+    """Light rejection on a graph with the hash set and 4-byte columns: the restatement's walks and edge ids."""
+    from mlx_cluster_b200 import ops
+    monkeypatch.setattr(ops, "_STEPS_PACKED_BYTES", 0)
+    rng = np.random.default_rng(17)
+    rowptr, col = random_csr(rng, 3000, 9.0, frac_isolated=0.2, symmetric=symmetric)
+    start = rng.integers(0, 3000, 5000).astype(np.int64)
+    graph = ops.WalkGraph(torch.from_numpy(rowptr).to(cuda), torch.from_numpy(col).to(cuda), symmetric=symmetric, edgeset=True)
+    graph.build_steps()
+    assert graph.steps is not None and graph.steps_bits == 0
+    _lib.set_tuning("n2v_team", -1)
+    try:
+        st = torch.from_numpy(start).to(cuda)
+        for L in (1, 7, 40):
+            want_n, want_e = oracle.node2vec_walk(rowptr, col, start, L, p, q, seed=3, return_edges=True)
+            n, e = rejection_sampling(None, None, st, L, p, q, graph=graph, seed=3, return_edges=True, check=True)
+            np.testing.assert_array_equal(n.cpu().numpy(), want_n)
+            np.testing.assert_array_equal(e.cpu().numpy(), want_e)
+            assert torch.equal(rejection_sampling(None, None, st, L, p, q, graph=graph, seed=3), n)
+    finally:
+        _lib.set_tuning("n2v_team", 0)
